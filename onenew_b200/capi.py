@@ -83,13 +83,15 @@ def check(rc):
 
 def shim_eval(op):
     """``eval`` of ``lib<Op>_cu.so`` -- the drop-in symbol."""
-    if op not in _shims:
+    fn = _shims.get(op)
+    if fn is None:
         lib()   # the shim links against the core library
         S = C.CDLL(shim_path(op))
-        S.eval.restype = C.c_int
-        S.eval.argtypes = [_BIP, _BIP, _BIP]
-        _shims[op] = S
-    return _shims[op].eval
+        fn = S.eval
+        fn.restype = C.c_int
+        fn.argtypes = [_BIP, _BIP, _BIP]
+        _shims[op] = fn
+    return fn
 
 
 class Context:
