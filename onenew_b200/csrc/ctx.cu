@@ -51,6 +51,56 @@ void *ws_alloc(one_ctx *c, size_t bytes)
     return c->ws + off;
 }
 
+// Status words are slots of one mapped page that lives as long as the process (pinning a page takes ~10 ms, too long
+// for every context); a context gives its slot back when it is released.  More contexts than slots: an error.
+static std::mutex g_slot_mu;
+static unsigned int *g_slots = nullptr;
+static bool g_slot_used[1024];
+
+static cudaError_t status_slot_take(unsigned int **host, unsigned int **dev)
+{
+    std::lock_guard<std::mutex> lk(g_slot_mu);
+    if (!g_slots) {
+        void *p = nullptr;
+        cudaError_t e = cudaHostAlloc(&p, sizeof(g_slot_used) * sizeof(unsigned int), cudaHostAllocMapped | cudaHostAllocPortable);
+        if (e != cudaSuccess) return e;
+        g_slots = static_cast<unsigned int *>(p);
+    }
+    for (size_t i = 0; i < sizeof(g_slot_used); ++i) {
+        if (g_slot_used[i]) continue;
+        void *d = nullptr;
+        cudaError_t e = cudaHostGetDevicePointer(&d, g_slots + i, 0);
+        if (e != cudaSuccess) return e;
+        g_slot_used[i] = true;
+        g_slots[i] = 0;
+        *host = g_slots + i;
+        *dev = static_cast<unsigned int *>(d);
+        return cudaSuccess;
+    }
+    return cudaErrorMemoryAllocation;
+}
+
+static void status_slot_give(const volatile unsigned int *host)
+{
+    if (!host) return;
+    std::lock_guard<std::mutex> lk(g_slot_mu);
+    g_slot_used[host - g_slots] = false;
+}
+
+int take_status(one_ctx *c)
+{
+    unsigned int st = 0;
+    if (c->status_host) {
+        st = *c->status_host;
+        if (st) *c->status_host = 0;
+    } else {
+        cudaError_t e = cudaMemcpy(&st, c->status_dev, sizeof(st), cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return cuda_fail(e, "status read");
+        if (st) cudaMemset(c->status_dev, 0, sizeof(st));
+    }
+    return st ? status_fail(st) : ONE_OK;
+}
+
 // ------------------------------------------------------------------ driver entry points
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                     const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -189,22 +239,23 @@ extern "C" int one_cuda_init(int device, size_t workspace_bytes, one_ctx **out)
         return fail(ONE_ERR_UNSUPPORTED, "device %d is sm_%d%d; this library holds sm_100a code only", device,
                     prop.major, prop.minor);
     one_ctx *c = new one_ctx();
+    unsigned int *status_host = nullptr;
     c->device = device;
     c->ws_bytes = workspace_bytes ? workspace_bytes : (size_t(256) << 20);
     if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaMalloc(&c->ws, c->ws_bytes)) != cudaSuccess ||
-        (e = cudaMalloc(&c->status_dev, sizeof(unsigned int))) != cudaSuccess ||
-        (e = cudaMemset(c->status_dev, 0, sizeof(unsigned int))) != cudaSuccess ||
+        (e = status_slot_take(&status_host, &c->status_dev)) != cudaSuccess ||
         (e = cudaMalloc(&c->ident16[0], 2 * 64 * 64 * 2)) != cudaSuccess) {
         int rc = cuda_fail(e, "one_cuda_init allocation");
         if (c->ws) cudaFree(c->ws);
-        if (c->status_dev) cudaFree(c->status_dev);
+        status_slot_give(status_host);
         if (c->ident16[0]) cudaFree(c->ident16[0]);
         if (c->stream) cudaStreamDestroy(c->stream);
         delete c;
         cudaSetDevice(prev);
         return rc;
     }
+    c->status_host = status_host;
     {   // 1.0 on the diagonal: 0x3F80 in bf16, 0x3C00 in fp16
         static uint16_t host[2][64 * 64];
         for (int f = 0; f < 2; ++f)
@@ -228,7 +279,7 @@ extern "C" int one_cuda_release(one_ctx *c)
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     cudaFree(c->ws);
-    cudaFree(c->status_dev);
+    status_slot_give(c->status_host);
     cudaFree(c->ident16[0]);
     cudaStreamDestroy(c->stream);
     delete c;
@@ -242,14 +293,7 @@ extern "C" int one_cuda_status(one_ctx *c)
     if (!c) return fail(ONE_ERR_BAD_ARG, "one_cuda_status: null context");
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "stream synchronise");
-    unsigned int st = 0;
-    if ((e = cudaMemcpy(&st, c->status_dev, sizeof(st), cudaMemcpyDeviceToHost)) != cudaSuccess)
-        return cuda_fail(e, "status read");
-    if (st) {
-        cudaMemset(c->status_dev, 0, sizeof(st));
-        return status_fail(st);
-    }
-    return ONE_OK;
+    return take_status(c);
 }
 
 extern "C" const char *one_cuda_last_error(void) { return g_err.c_str(); }

@@ -15,7 +15,11 @@ struct one_ctx {
     uint8_t *ws = nullptr;      // scratch workspace
     size_t ws_bytes = 0;
     size_t ws_off = 0;          // bump offset of the call in progress
+    // Status word the kernels report through: pinned host memory mapped into the device's address space, so that the
+    // host reads it after a stream synchronisation without a copy (~8 us of every synchronous call).  A context whose
+    // word lives in device memory (the allocation-free Conv) has no host view of it: status_host is null then.
     unsigned int *status_dev = nullptr;
+    volatile unsigned int *status_host = nullptr;
     bool allow_split = true;    // split-K contractions may take scratch for their partial sums
     void *ident16[2] = {nullptr, nullptr};   // 64 x 64 identity matrices in bf16 [0] and fp16 [1] (residual added by the tensor core)
 };
@@ -26,6 +30,7 @@ void set_error(const char *fmt, ...);
 int fail(int code, const char *fmt, ...);          // set_error + return code
 int cuda_fail(cudaError_t e, const char *what);    // ONE_ERR_CUDA with the runtime's text
 int status_fail(unsigned int status_word);         // the error a non-zero device status word stands for
+int take_status(one_ctx *c);                       // after a synchronisation: read and clear the word, 0 or its error
 
 // Workspace: reset at the start of every operator call, 256-byte aligned blocks.
 inline void ws_reset(one_ctx *c) { c->ws_off = 0; }

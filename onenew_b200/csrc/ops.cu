@@ -633,14 +633,7 @@ int finish_sync(one_ctx *ctx, cudaStream_t stream)
 {
     cudaError_t e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return cuda_fail(e, "stream synchronise");
-    unsigned int st = 0;
-    if ((e = cudaMemcpy(&st, ctx->status_dev, sizeof(st), cudaMemcpyDeviceToHost)) != cudaSuccess)
-        return cuda_fail(e, "status read");
-    if (st) {
-        cudaMemset(ctx->status_dev, 0, sizeof(st));
-        return status_fail(st);
-    }
-    return ONE_OK;
+    return take_status(ctx);
 }
 
 // int8 de-quantisation coefficients exactly as the reference forms them:
