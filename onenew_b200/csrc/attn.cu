@@ -32,6 +32,7 @@
 
 #include "../../include/one_cuda.h"
 #include "ctx.h"
+#include "launch.cuh"
 #include "sm100_prims.cuh"
 
 namespace one {
@@ -121,6 +122,8 @@ attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(tmem_slot);
+    pdl_launch_dependents();   // everything above touched nothing an earlier kernel writes
+    pdl_wait();
 
     bool v_issued = false;
     if (warp == 4) {
@@ -352,7 +355,7 @@ extern "C" int one_cuda_attention(one_ctx *ctx, const float *qkv, float *out, in
     }
     const long long tiles = (long long)batch * heads * p.m_tiles;
     if (tiles > 0x7fffffffLL) return fail(ONE_ERR_BAD_SHAPE, "attention: too many tiles");
-    attn_kernel<<<(unsigned)tiles, ATTN_THREADS, smem, st>>>(tmQ, tmK, tmV, tmO, p);
+    launch_k(attn_kernel, (unsigned)tiles, ATTN_THREADS, smem, st, tmQ, tmK, tmV, tmO, p);
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ONE_OK : cuda_fail(e, "attention launch");

@@ -5,6 +5,7 @@
 // int8 path (conv.c:961-973).
 #include "glue.cuh"
 #include "ctx.h"
+#include "launch.cuh"
 #include "act.cuh"
 
 #include <cuda_bf16.h>
@@ -54,6 +55,7 @@ template <typename T>
 __global__ void k_nchw_to_nhwc(const float *__restrict__ x, T *__restrict__ y, int C, int HW, int round_tf32,
                                float inv_scale)
 {
+    pdl_entry(x);
     __shared__ float tile[32][33];
     const int n = blockIdx.z;
     const int c0 = blockIdx.y * 32, p0 = blockIdx.x * 32;
@@ -73,6 +75,7 @@ __global__ void k_nchw_to_nhwc(const float *__restrict__ x, T *__restrict__ y, i
 template <typename T>
 __global__ void k_nhwc_to_nchw(const T *__restrict__ x, float *__restrict__ y, int C, int HW)
 {
+    pdl_entry(x);
     __shared__ float tile[32][33];
     const int n = blockIdx.z;
     const int c0 = blockIdx.y * 32, p0 = blockIdx.x * 32;
@@ -94,10 +97,10 @@ cudaError_t nchw_to_nhwc(const float *x, void *y, int N, int C, int HW, int dt, 
 {
     if (N <= 0 || C <= 0 || HW <= 0) return cudaSuccess;
     dim3 grid((HW + 31) / 32, (C + 31) / 32, N), block(32, 8);
-    if (dt == DT_F32) k_nchw_to_nhwc<float><<<grid, block, 0, s>>>(x, (float *)y, C, HW, round_tf32, inv_scale);
-    else if (dt == DT_BF16) k_nchw_to_nhwc<__nv_bfloat16><<<grid, block, 0, s>>>(x, (__nv_bfloat16 *)y, C, HW, 0, inv_scale);
-    else if (dt == DT_F16) k_nchw_to_nhwc<__half><<<grid, block, 0, s>>>(x, (__half *)y, C, HW, 0, inv_scale);
-    else k_nchw_to_nhwc<int8_t><<<grid, block, 0, s>>>(x, (int8_t *)y, C, HW, 0, inv_scale);
+    if (dt == DT_F32) launch_k(k_nchw_to_nhwc<float>, grid, block, 0, s, x, (float *)y, C, HW, round_tf32, inv_scale);
+    else if (dt == DT_BF16) launch_k(k_nchw_to_nhwc<__nv_bfloat16>, grid, block, 0, s, x, (__nv_bfloat16 *)y, C, HW, 0, inv_scale);
+    else if (dt == DT_F16) launch_k(k_nchw_to_nhwc<__half>, grid, block, 0, s, x, (__half *)y, C, HW, 0, inv_scale);
+    else launch_k(k_nchw_to_nhwc<int8_t>, grid, block, 0, s, x, (int8_t *)y, C, HW, 0, inv_scale);
     count_launch();
     return cudaGetLastError();
 }
@@ -106,10 +109,10 @@ cudaError_t nhwc_to_nchw(const void *x, float *y, int N, int C, int HW, int dt, 
 {
     if (N <= 0 || C <= 0 || HW <= 0) return cudaSuccess;
     dim3 grid((HW + 31) / 32, (C + 31) / 32, N), block(32, 8);
-    if (dt == DT_F32) k_nhwc_to_nchw<float><<<grid, block, 0, s>>>((const float *)x, y, C, HW);
-    else if (dt == DT_BF16) k_nhwc_to_nchw<__nv_bfloat16><<<grid, block, 0, s>>>((const __nv_bfloat16 *)x, y, C, HW);
-    else if (dt == DT_F16) k_nhwc_to_nchw<__half><<<grid, block, 0, s>>>((const __half *)x, y, C, HW);
-    else if (dt == DT_S8) k_nhwc_to_nchw<int8_t><<<grid, block, 0, s>>>((const int8_t *)x, y, C, HW);   // the quantised integers as floats
+    if (dt == DT_F32) launch_k(k_nhwc_to_nchw<float>, grid, block, 0, s, (const float *)x, y, C, HW);
+    else if (dt == DT_BF16) launch_k(k_nhwc_to_nchw<__nv_bfloat16>, grid, block, 0, s, (const __nv_bfloat16 *)x, y, C, HW);
+    else if (dt == DT_F16) launch_k(k_nhwc_to_nchw<__half>, grid, block, 0, s, (const __half *)x, y, C, HW);
+    else if (dt == DT_S8) launch_k(k_nhwc_to_nchw<int8_t>, grid, block, 0, s, (const int8_t *)x, y, C, HW);   // the quantised integers as floats
     else return cudaErrorInvalidValue;
     count_launch();
     return cudaGetLastError();
@@ -120,6 +123,7 @@ template <typename T>
 __global__ void k_pack_conv_weight(const void *__restrict__ w, T *__restrict__ out, int OC, int C, int KH, int KW,
                                    int Kp, int src_is_s8)
 {
+    pdl_entry(w);
     const long long total = (long long)OC * Kp;
     const int K = C * KH * KW;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -146,10 +150,10 @@ cudaError_t pack_conv_weight(const void *w, void *out, int OC, int C, int KH, in
     const long long total = (long long)OC * Kp;
     const int block = 256;
     const int grid = (int)((total + block - 1) / block > 4096 ? 4096 : (total + block - 1) / block);
-    if (dt == DT_F32) k_pack_conv_weight<float><<<grid, block, 0, s>>>(w, (float *)out, OC, C, KH, KW, Kp, src_is_s8);
-    else if (dt == DT_BF16) k_pack_conv_weight<__nv_bfloat16><<<grid, block, 0, s>>>(w, (__nv_bfloat16 *)out, OC, C, KH, KW, Kp, src_is_s8);
-    else if (dt == DT_F16) k_pack_conv_weight<__half><<<grid, block, 0, s>>>(w, (__half *)out, OC, C, KH, KW, Kp, src_is_s8);
-    else k_pack_conv_weight<int8_t><<<grid, block, 0, s>>>(w, (int8_t *)out, OC, C, KH, KW, Kp, src_is_s8);
+    if (dt == DT_F32) launch_k(k_pack_conv_weight<float>, grid, block, 0, s, w, (float *)out, OC, C, KH, KW, Kp, src_is_s8);
+    else if (dt == DT_BF16) launch_k(k_pack_conv_weight<__nv_bfloat16>, grid, block, 0, s, w, (__nv_bfloat16 *)out, OC, C, KH, KW, Kp, src_is_s8);
+    else if (dt == DT_F16) launch_k(k_pack_conv_weight<__half>, grid, block, 0, s, w, (__half *)out, OC, C, KH, KW, Kp, src_is_s8);
+    else launch_k(k_pack_conv_weight<int8_t>, grid, block, 0, s, w, (int8_t *)out, OC, C, KH, KW, Kp, src_is_s8);
     count_launch();
     return cudaGetLastError();
 }
@@ -157,6 +161,7 @@ cudaError_t pack_conv_weight(const void *w, void *out, int OC, int C, int KH, in
 template <typename T>
 __global__ void k_pack_rows(const float *__restrict__ a, T *__restrict__ out, long long R, int K, int Kp)
 {
+    pdl_entry(a);
     const long long total = R * Kp;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long r = i / Kp;
@@ -171,9 +176,9 @@ cudaError_t pack_rows(const float *a, void *out, long long R, int K, int Kp, int
     if (total <= 0) return cudaSuccess;
     const int block = 256;
     const int grid = (int)((total + block - 1) / block > 148 * 16 ? 148 * 16 : (total + block - 1) / block);
-    if (dt == DT_F32) k_pack_rows<float><<<grid, block, 0, s>>>(a, (float *)out, R, K, Kp);
-    else if (dt == DT_BF16) k_pack_rows<__nv_bfloat16><<<grid, block, 0, s>>>(a, (__nv_bfloat16 *)out, R, K, Kp);
-    else if (dt == DT_F16) k_pack_rows<__half><<<grid, block, 0, s>>>(a, (__half *)out, R, K, Kp);
+    if (dt == DT_F32) launch_k(k_pack_rows<float>, grid, block, 0, s, a, (float *)out, R, K, Kp);
+    else if (dt == DT_BF16) launch_k(k_pack_rows<__nv_bfloat16>, grid, block, 0, s, a, (__nv_bfloat16 *)out, R, K, Kp);
+    else if (dt == DT_F16) launch_k(k_pack_rows<__half>, grid, block, 0, s, a, (__half *)out, R, K, Kp);
     else return cudaErrorInvalidValue;
     count_launch();
     return cudaGetLastError();
@@ -182,6 +187,7 @@ cudaError_t pack_rows(const float *a, void *out, long long R, int K, int Kp, int
 template <typename T>
 __global__ void k_pack_transposed(const float *__restrict__ b, T *__restrict__ out, int K, int N, int Kp)
 {
+    pdl_entry(b);
     __shared__ float tile[32][33];
     const int bi = blockIdx.z;
     const int k0 = blockIdx.y * 32, n0 = blockIdx.x * 32;
@@ -202,9 +208,9 @@ cudaError_t pack_transposed(const float *b, void *out, int batch, int K, int N, 
 {
     if (batch <= 0 || K <= 0 || N <= 0) return cudaSuccess;
     dim3 grid((N + 31) / 32, (Kp + 31) / 32, batch), block(32, 8);
-    if (dt == DT_F32) k_pack_transposed<float><<<grid, block, 0, s>>>(b, (float *)out, K, N, Kp);
-    else if (dt == DT_BF16) k_pack_transposed<__nv_bfloat16><<<grid, block, 0, s>>>(b, (__nv_bfloat16 *)out, K, N, Kp);
-    else if (dt == DT_F16) k_pack_transposed<__half><<<grid, block, 0, s>>>(b, (__half *)out, K, N, Kp);
+    if (dt == DT_F32) launch_k(k_pack_transposed<float>, grid, block, 0, s, b, (float *)out, K, N, Kp);
+    else if (dt == DT_BF16) launch_k(k_pack_transposed<__nv_bfloat16>, grid, block, 0, s, b, (__nv_bfloat16 *)out, K, N, Kp);
+    else if (dt == DT_F16) launch_k(k_pack_transposed<__half>, grid, block, 0, s, b, (__half *)out, K, N, Kp);
     else return cudaErrorInvalidValue;
     count_launch();
     return cudaGetLastError();
@@ -218,6 +224,7 @@ template <typename T>
 __global__ void k_patch_pack(const float *__restrict__ x, T *__restrict__ out, long long M, int C, int H, int W, int KH, int KW,
                              int OH, int OW, int Kp)
 {
+    pdl_entry(x);
     const int K = C * KH * KW, k4n = Kp >> 2;
     const long long total = M * k4n;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -249,9 +256,9 @@ cudaError_t patch_pack(const float *x, void *out, int N, int C, int H, int W, in
     if (total <= 0) return cudaSuccess;
     const int block = 256;
     const int grid = (int)((total + block - 1) / block > 148 * 32 ? 148 * 32 : (total + block - 1) / block);
-    if (dt == DT_F32) k_patch_pack<float><<<grid, block, 0, s>>>(x, (float *)out, M, C, H, W, KH, KW, OH, OW, Kp);
-    else if (dt == DT_BF16) k_patch_pack<__nv_bfloat16><<<grid, block, 0, s>>>(x, (__nv_bfloat16 *)out, M, C, H, W, KH, KW, OH, OW, Kp);
-    else if (dt == DT_F16) k_patch_pack<__half><<<grid, block, 0, s>>>(x, (__half *)out, M, C, H, W, KH, KW, OH, OW, Kp);
+    if (dt == DT_F32) launch_k(k_patch_pack<float>, grid, block, 0, s, x, (float *)out, M, C, H, W, KH, KW, OH, OW, Kp);
+    else if (dt == DT_BF16) launch_k(k_patch_pack<__nv_bfloat16>, grid, block, 0, s, x, (__nv_bfloat16 *)out, M, C, H, W, KH, KW, OH, OW, Kp);
+    else if (dt == DT_F16) launch_k(k_patch_pack<__half>, grid, block, 0, s, x, (__half *)out, M, C, H, W, KH, KW, OH, OW, Kp);
     else return cudaErrorInvalidValue;
     count_launch();
     return cudaGetLastError();
@@ -265,6 +272,7 @@ __global__ void k_im2col_pack(const TS *__restrict__ x, TD *__restrict__ out, in
                               int OH, int OW, int stride_w, int stride_h, int pad_t, int pad_l, int Kp, int src_nhwc,
                               float inv_scale)
 {
+    pdl_entry(x);
     const long long M = (long long)N * OH * OW;
     const long long total = M * Kp;
     const int K = C * KH * KW;
@@ -303,7 +311,7 @@ cudaError_t im2col_pack(const void *x, void *out, int N, int C, int H, int W, in
     long long g = (total + block - 1) / block;
     const int grid = (int)(g > 148LL * 32 ? 148LL * 32 : g);
 #define ONE_I2C(TS, TD)                                                                                      \
-    k_im2col_pack<TS, TD><<<grid, block, 0, s>>>((const TS *)x, (TD *)out, N, C, H, W, KH, KW, OH, OW, stride_w, \
+    launch_k(k_im2col_pack<TS, TD>, grid, block, 0, s, (const TS *)x, (TD *)out, N, C, H, W, KH, KW, OH, OW, stride_w, \
                                                  stride_h, pad_t, pad_l, Kp, src_nhwc, inv_scale)
     if (src_dt == DT_F32 && dt == DT_F32) ONE_I2C(float, float);
     else if (src_dt == DT_F32 && dt == DT_BF16) ONE_I2C(float, __nv_bfloat16);
@@ -327,6 +335,7 @@ cudaError_t im2col_pack(const void *x, void *out, int N, int C, int H, int W, in
 template <typename T, int C, int BW>
 __global__ void k_s2d_pack(const float *__restrict__ x, T *__restrict__ out, int N, int H, int W, int Hs, int Ws, float inv_scale)
 {
+    pdl_entry(x);
     constexpr int CB = 2 * BW * C * (int)sizeof(T);
     constexpr int CP = (CB <= 32 ? 32 : (CB <= 64 ? 64 : 128)) / (int)sizeof(T);   // must match s2d_plan
     constexpr int NV = CP * (int)sizeof(T) / 16;
@@ -385,7 +394,7 @@ cudaError_t s2d_pack(const float *x, void *out, int N, int C, int H, int W, int 
     const int block = 256;
     long long g = (total + block - 1) / block;
     const int grid = (int)(g > 148LL * 32 ? 148LL * 32 : g);
-#define ONE_S2D(T, CC, BB) k_s2d_pack<T, CC, BB><<<grid, block, 0, s>>>(x, (T *)out, N, H, W, Hs, Ws, inv_scale)
+#define ONE_S2D(T, CC, BB) launch_k(k_s2d_pack<T, CC, BB>, grid, block, 0, s, x, (T *)out, N, H, W, Hs, Ws, inv_scale)
 #define ONE_S2D_C(T)                                                                                      \
     if (bw == 4) {                                                                                        \
         switch (C) {                                                                                      \
@@ -413,6 +422,7 @@ template <typename T>
 __global__ void k_pack_conv_weight_s2d(const void *__restrict__ w, T *__restrict__ out, int OC, int C, int KH, int KW, int KH2,
                                        int KW2, int eh, int ew, int Cp, int bwid, int src_is_s8)
 {
+    pdl_entry(w);
     const int pitch = KH2 * KW2 * Cp;
     const long long total = (long long)OC * pitch;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -445,10 +455,10 @@ cudaError_t pack_conv_weight_s2d(const void *w, void *out, int OC, int C, int KH
     const long long total = (long long)OC * KH2 * KW2 * Cp;
     const int block = 256;
     const int grid = (int)((total + block - 1) / block > 4096 ? 4096 : (total + block - 1) / block);
-    if (dt == DT_F32) k_pack_conv_weight_s2d<float><<<grid, block, 0, s>>>(w, (float *)out, OC, C, KH, KW, KH2, KW2, eh, ew, Cp, bw, src_is_s8);
-    else if (dt == DT_BF16) k_pack_conv_weight_s2d<__nv_bfloat16><<<grid, block, 0, s>>>(w, (__nv_bfloat16 *)out, OC, C, KH, KW, KH2, KW2, eh, ew, Cp, bw, src_is_s8);
-    else if (dt == DT_F16) k_pack_conv_weight_s2d<__half><<<grid, block, 0, s>>>(w, (__half *)out, OC, C, KH, KW, KH2, KW2, eh, ew, Cp, bw, src_is_s8);
-    else k_pack_conv_weight_s2d<int8_t><<<grid, block, 0, s>>>(w, (int8_t *)out, OC, C, KH, KW, KH2, KW2, eh, ew, Cp, bw, src_is_s8);
+    if (dt == DT_F32) launch_k(k_pack_conv_weight_s2d<float>, grid, block, 0, s, w, (float *)out, OC, C, KH, KW, KH2, KW2, eh, ew, Cp, bw, src_is_s8);
+    else if (dt == DT_BF16) launch_k(k_pack_conv_weight_s2d<__nv_bfloat16>, grid, block, 0, s, w, (__nv_bfloat16 *)out, OC, C, KH, KW, KH2, KW2, eh, ew, Cp, bw, src_is_s8);
+    else if (dt == DT_F16) launch_k(k_pack_conv_weight_s2d<__half>, grid, block, 0, s, w, (__half *)out, OC, C, KH, KW, KH2, KW2, eh, ew, Cp, bw, src_is_s8);
+    else launch_k(k_pack_conv_weight_s2d<int8_t>, grid, block, 0, s, w, (int8_t *)out, OC, C, KH, KW, KH2, KW2, eh, ew, Cp, bw, src_is_s8);
     count_launch();
     return cudaGetLastError();
 }
@@ -462,6 +472,7 @@ __global__ void k_dwconv_nchw(const float *__restrict__ x, const float *__restri
                               float *__restrict__ y, int N, int C, int H, int W, int OH, int OW, int KH, int KW, int sx, int sy,
                               int pt, int pl, int act, float p0, float p1, const float *__restrict__ lut)
 {
+    pdl_entry(x, w, bias, lut);
     const long long total = (long long)N * C * OH * OW;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int ow = (int)(i % OW);
@@ -495,6 +506,7 @@ __global__ void k_dwconv_s8_nchw(const float *__restrict__ x, const int8_t *__re
                                  int KH, int KW, int sx, int sy, int pad, float in_scale, float inv_scale, int act, float p0,
                                  float p1, const float *__restrict__ lut)
 {
+    pdl_entry(x, w, bias, aux, lut);
     const long long total = (long long)N * C * OH * OW;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int ow = (int)(i % OW);
@@ -533,7 +545,7 @@ cudaError_t dwconv_nchw(const float *x, const float *w, const float *bias, float
 {
     const long long total = (long long)N * C * OH * OW;
     if (total <= 0) return cudaSuccess;
-    k_dwconv_nchw<<<dw_grid(total, 256), 256, 0, s>>>(x, w, bias, y, N, C, H, W, OH, OW, KH, KW, sx, sy, pt, pl, act, p0, p1, lut);
+    launch_k(k_dwconv_nchw, dw_grid(total, 256), 256, 0, s, x, w, bias, y, N, C, H, W, OH, OW, KH, KW, sx, sy, pt, pl, act, p0, p1, lut);
     count_launch();
     return cudaGetLastError();
 }
@@ -544,7 +556,7 @@ cudaError_t dwconv_s8_nchw(const float *x, const int8_t *w, const int *bias, con
 {
     const long long total = (long long)N * C * OH * OW;
     if (total <= 0) return cudaSuccess;
-    k_dwconv_s8_nchw<<<dw_grid(total, 256), 256, 0, s>>>(x, w, bias, aux, y, N, C, H, W, OH, OW, KH, KW, sx, sy, pad, in_scale,
+    launch_k(k_dwconv_s8_nchw, dw_grid(total, 256), 256, 0, s, x, w, bias, aux, y, N, C, H, W, OH, OW, KH, KW, sx, sy, pad, in_scale,
                                                          1.0f / in_scale, act, p0, p1, lut);
     count_launch();
     return cudaGetLastError();
@@ -552,19 +564,21 @@ cudaError_t dwconv_s8_nchw(const float *x, const int8_t *w, const int *bias, con
 
 __global__ void k_cast_s32_f32(const int *__restrict__ x, float *__restrict__ y, long long n)
 {
+    pdl_entry(x);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) y[i] = (float)x[i];
 }
 
 cudaError_t cast_s32_f32(const int *x, float *y, long long n, cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
-    k_cast_s32_f32<<<(int)((n + 255) / 256 > 1024 ? 1024 : (n + 255) / 256), 256, 0, s>>>(x, y, n);
+    launch_k(k_cast_s32_f32, (int)((n + 255) / 256 > 1024 ? 1024 : (n + 255) / 256), 256, 0, s, x, y, n);
     count_launch();
     return cudaGetLastError();
 }
 
 __global__ void k_quantize_s8(const float *__restrict__ x, int8_t *__restrict__ q, long long n, float inv_scale)
 {
+    pdl_entry(x);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         q[i] = q8(x[i], inv_scale);
 }
@@ -574,7 +588,7 @@ cudaError_t quantize_s8(const float *x, int8_t *q, long long n, float inv_scale,
     if (n <= 0) return cudaSuccess;
     const int block = 256;
     long long g = (n + block - 1) / block;
-    k_quantize_s8<<<(int)(g > 148LL * 16 ? 148LL * 16 : g), block, 0, s>>>(x, q, n, inv_scale);
+    launch_k(k_quantize_s8, (int)(g > 148LL * 16 ? 148LL * 16 : g), block, 0, s, x, q, n, inv_scale);
     count_launch();
     return cudaGetLastError();
 }

@@ -25,13 +25,13 @@
 #include "sm100_prims.cuh"
 #include "act.cuh"
 #include "ctx.h"
+#include "launch.cuh"
 
 #include <cuda_bf16.h>
 #include "h16.cuh"
 #include <string.h>
 
 #include <atomic>
-#include <utility>
 
 namespace one {
 
@@ -284,9 +284,10 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     // completed and its writes are visible.  Every thread executes the wait, so each role's global
     // accesses are ordered after it.  The next kernel may start its own prologue right away; it cannot
     // touch data before its own wait, which in turn covers this whole grid.
+    // (The release of the next launch comes first: its blocks then do their own set-up while this one waits.)
     if (p.pdl) {
-        pdl_wait();
         pdl_launch_dependents();
+        pdl_wait();
     }
 
     long long issued = 0;   // producer: ring stages whose loads were issued (ring position)
@@ -1041,8 +1042,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const SplitKReduceParams p, int pdl)
 {
     if (pdl) {
-        pdl_wait();
         pdl_launch_dependents();
+        pdl_wait();
     }
     const bool out16 = out_is_16(p.out_mode), f16 = p.out_mode == OUT_F16;
     float vmax = 0.f;
@@ -1136,37 +1137,6 @@ int get_epilogue_mode() { return g_epi_mode.load(std::memory_order_relaxed); }
 void set_epilogue_mode(int bits) { g_epi_mode.store(bits & 15, std::memory_order_relaxed); }
 void set_pdl(int on) { g_pdl.store(on ? 1 : 0, std::memory_order_relaxed); }
 int get_pdl() { return g_pdl.load(std::memory_order_relaxed); }
-
-// Launch with the programmatic-stream-serialisation attribute when `pdl` (the kernel may be scheduled
-// before the previous kernel on the stream has finished and orders itself with griddepcontrol.wait) and as
-// clusters of `cluster` CTAs when that is above 1.
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_ex(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl, int cluster, Args &&...args)
-{
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    int n = 0;
-    if (pdl) {
-        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n].val.programmaticStreamSerializationAllowed = 1;
-        ++n;
-    }
-    if (cluster > 1) {
-        attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = (unsigned)cluster;
-        attr[n].val.clusterDim.y = 1;
-        attr[n].val.clusterDim.z = 1;
-        ++n;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
 
 static int sm_count_of(int dev)
 {

@@ -15,6 +15,7 @@
 
 #include "../../include/one_glue.h"
 #include "ctx.h"
+#include "launch.cuh"
 #include "glue.cuh"
 
 using namespace one;
@@ -94,6 +95,7 @@ template <typename T, bool VEC>
 __global__ void k_maxpool_nhwc(const T *__restrict__ x, T *__restrict__ y, int N, int H, int W, int C, int OH, int OW,
                                int kh, int kw, int sh, int sw, int pad)
 {
+    pdl_entry(x);
     constexpr int V = VEC ? Vec<T>::N : 1;
     const int cv = C / V;
     const long long total = (long long)N * OH * OW * cv;
@@ -136,6 +138,7 @@ __global__ void k_maxpool_nhwc(const T *__restrict__ x, T *__restrict__ y, int N
 template <typename T>
 __global__ void k_maxpool3x3s2_nhwc(const T *__restrict__ x, T *__restrict__ y, int N, int H, int W, int C, int OH, int OW, int pad)
 {
+    pdl_entry(x);
     constexpr int V = Vec<T>::N;
     const int cv = C / V;
     const int owp = (OW + 1) / 2;
@@ -199,6 +202,7 @@ template <typename T2>
 __global__ void k_maxpool3x3s2_nhwc_p16(const uint4 *__restrict__ x, uint4 *__restrict__ y, int N, int H, int W, int C, int OH, int OW, int pad,
                                         uint32_t minus_inf2)
 {
+    pdl_entry(x);
     const int cv = C / 8;
     const int owp = (OW + 1) / 2;
     const long long total = (long long)N * OH * owp * cv;
@@ -235,6 +239,7 @@ template <typename T, bool VEC>
 __global__ void k_add_relu(const T *__restrict__ a, const T *__restrict__ b, T *__restrict__ y, long long n, int has_b,
                            int relu)
 {
+    pdl_entry(a, b);
     constexpr int V = VEC ? Vec<T>::N : 1;
     const long long nv = n / V;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
@@ -261,6 +266,7 @@ __global__ void k_add_relu(const T *__restrict__ a, const T *__restrict__ b, T *
 template <typename T>
 __global__ void k_gap_nhwc(const T *__restrict__ x, T *__restrict__ y, int N, int HW, int C)
 {
+    pdl_entry(x);
     const long long total = (long long)N * C;
     const float coeff = 1.0f / (float)HW;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -278,6 +284,7 @@ __global__ void k_gap_nhwc(const T *__restrict__ x, T *__restrict__ y, int N, in
 template <typename T>
 __global__ void k_gap_nhwc_vec(const T *__restrict__ x, T *__restrict__ y, int N, int HW, int C)
 {
+    pdl_entry(x);
     constexpr int V = Vec<T>::N;
     const int cv = C / V;
     const long long total = (long long)N * cv;
@@ -314,6 +321,7 @@ __global__ void k_gap_nhwc_vec(const T *__restrict__ x, T *__restrict__ y, int N
 template <typename TI, typename TO>
 __global__ void k_cast(const TI *__restrict__ x, TO *__restrict__ y, long long n)
 {
+    pdl_entry(x);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         Vec<TO>::st1(y + i, Vec<TI>::ld1(x + i));
 }
@@ -342,23 +350,23 @@ extern "C" int one_glue_maxpool_nhwc(const void *x, void *y, int dtype, int N, i
         const bool vec = (C % 4 == 0) && aligned16(x) && aligned16(y);
         const long long work = (long long)N * OH * OW * (vec ? C / 4 : C);
         if (vec && kh == 3 && kw == 3 && sh == 2 && sw == 2)
-            k_maxpool3x3s2_nhwc<float><<<grid_for((long long)N * OH * ((OW + 1) / 2) * (C / 4), block), block, 0, st>>>((const float *)x, (float *)y, N, H, W, C, OH, OW, pad);
-        else if (vec) k_maxpool_nhwc<float, true><<<grid_for(work, block), block, 0, st>>>((const float *)x, (float *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
-        else k_maxpool_nhwc<float, false><<<grid_for(work, block), block, 0, st>>>((const float *)x, (float *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
+            launch_k(k_maxpool3x3s2_nhwc<float>, grid_for((long long)N * OH * ((OW + 1) / 2) * (C / 4), block), block, 0, st, (const float *)x, (float *)y, N, H, W, C, OH, OW, pad);
+        else if (vec) launch_k(k_maxpool_nhwc<float, true>, grid_for(work, block), block, 0, st, (const float *)x, (float *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
+        else launch_k(k_maxpool_nhwc<float, false>, grid_for(work, block), block, 0, st, (const float *)x, (float *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
     } else if (dtype == DT_BF16) {
         const bool vec = (C % 8 == 0) && aligned16(x) && aligned16(y);
         const long long work = (long long)N * OH * OW * (vec ? C / 8 : C);
         if (vec && kh == 3 && kw == 3 && sh == 2 && sw == 2)
-            k_maxpool3x3s2_nhwc_p16<__nv_bfloat162><<<grid_for((long long)N * OH * ((OW + 1) / 2) * (C / 8), block), block, 0, st>>>((const uint4 *)x, (uint4 *)y, N, H, W, C, OH, OW, pad, 0xFF80FF80u);
-        else if (vec) k_maxpool_nhwc<__nv_bfloat16, true><<<grid_for(work, block), block, 0, st>>>((const __nv_bfloat16 *)x, (__nv_bfloat16 *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
-        else k_maxpool_nhwc<__nv_bfloat16, false><<<grid_for(work, block), block, 0, st>>>((const __nv_bfloat16 *)x, (__nv_bfloat16 *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
+            launch_k(k_maxpool3x3s2_nhwc_p16<__nv_bfloat162>, grid_for((long long)N * OH * ((OW + 1) / 2) * (C / 8), block), block, 0, st, (const uint4 *)x, (uint4 *)y, N, H, W, C, OH, OW, pad, 0xFF80FF80u);
+        else if (vec) launch_k(k_maxpool_nhwc<__nv_bfloat16, true>, grid_for(work, block), block, 0, st, (const __nv_bfloat16 *)x, (__nv_bfloat16 *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
+        else launch_k(k_maxpool_nhwc<__nv_bfloat16, false>, grid_for(work, block), block, 0, st, (const __nv_bfloat16 *)x, (__nv_bfloat16 *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
     } else if (dtype == DT_F16) {
         const bool vec = (C % 8 == 0) && aligned16(x) && aligned16(y);
         const long long work = (long long)N * OH * OW * (vec ? C / 8 : C);
         if (vec && kh == 3 && kw == 3 && sh == 2 && sw == 2)
-            k_maxpool3x3s2_nhwc_p16<__half2><<<grid_for((long long)N * OH * ((OW + 1) / 2) * (C / 8), block), block, 0, st>>>((const uint4 *)x, (uint4 *)y, N, H, W, C, OH, OW, pad, 0xFC00FC00u);
-        else if (vec) k_maxpool_nhwc<__half, true><<<grid_for(work, block), block, 0, st>>>((const __half *)x, (__half *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
-        else k_maxpool_nhwc<__half, false><<<grid_for(work, block), block, 0, st>>>((const __half *)x, (__half *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
+            launch_k(k_maxpool3x3s2_nhwc_p16<__half2>, grid_for((long long)N * OH * ((OW + 1) / 2) * (C / 8), block), block, 0, st, (const uint4 *)x, (uint4 *)y, N, H, W, C, OH, OW, pad, 0xFC00FC00u);
+        else if (vec) launch_k(k_maxpool_nhwc<__half, true>, grid_for(work, block), block, 0, st, (const __half *)x, (__half *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
+        else launch_k(k_maxpool_nhwc<__half, false>, grid_for(work, block), block, 0, st, (const __half *)x, (__half *)y, N, H, W, C, OH, OW, kh, kw, sh, sw, pad);
     } else return fail(ONE_ERR_UNSUPPORTED, "MaxPool: dtype %d", dtype);
     count_launch();
     cudaError_t e = cudaGetLastError();
@@ -374,16 +382,16 @@ extern "C" int one_glue_add_relu(const void *a, const void *b, void *y, int dtyp
     const int has_b = b != nullptr;
     if (dtype == DT_F32) {
         const bool vec = (n % 4 == 0) && aligned16(a) && aligned16(y) && (!b || aligned16(b));
-        if (vec) k_add_relu<float, true><<<grid_for(n / 4, block), block, 0, st>>>((const float *)a, (const float *)b, (float *)y, n, has_b, relu);
-        else k_add_relu<float, false><<<grid_for(n, block), block, 0, st>>>((const float *)a, (const float *)b, (float *)y, n, has_b, relu);
+        if (vec) launch_k(k_add_relu<float, true>, grid_for(n / 4, block), block, 0, st, (const float *)a, (const float *)b, (float *)y, n, has_b, relu);
+        else launch_k(k_add_relu<float, false>, grid_for(n, block), block, 0, st, (const float *)a, (const float *)b, (float *)y, n, has_b, relu);
     } else if (dtype == DT_BF16) {
         const bool vec = (n % 8 == 0) && aligned16(a) && aligned16(y) && (!b || aligned16(b));
-        if (vec) k_add_relu<__nv_bfloat16, true><<<grid_for(n / 8, block), block, 0, st>>>((const __nv_bfloat16 *)a, (const __nv_bfloat16 *)b, (__nv_bfloat16 *)y, n, has_b, relu);
-        else k_add_relu<__nv_bfloat16, false><<<grid_for(n, block), block, 0, st>>>((const __nv_bfloat16 *)a, (const __nv_bfloat16 *)b, (__nv_bfloat16 *)y, n, has_b, relu);
+        if (vec) launch_k(k_add_relu<__nv_bfloat16, true>, grid_for(n / 8, block), block, 0, st, (const __nv_bfloat16 *)a, (const __nv_bfloat16 *)b, (__nv_bfloat16 *)y, n, has_b, relu);
+        else launch_k(k_add_relu<__nv_bfloat16, false>, grid_for(n, block), block, 0, st, (const __nv_bfloat16 *)a, (const __nv_bfloat16 *)b, (__nv_bfloat16 *)y, n, has_b, relu);
     } else if (dtype == DT_F16) {
         const bool vec = (n % 8 == 0) && aligned16(a) && aligned16(y) && (!b || aligned16(b));
-        if (vec) k_add_relu<__half, true><<<grid_for(n / 8, block), block, 0, st>>>((const __half *)a, (const __half *)b, (__half *)y, n, has_b, relu);
-        else k_add_relu<__half, false><<<grid_for(n, block), block, 0, st>>>((const __half *)a, (const __half *)b, (__half *)y, n, has_b, relu);
+        if (vec) launch_k(k_add_relu<__half, true>, grid_for(n / 8, block), block, 0, st, (const __half *)a, (const __half *)b, (__half *)y, n, has_b, relu);
+        else launch_k(k_add_relu<__half, false>, grid_for(n, block), block, 0, st, (const __half *)a, (const __half *)b, (__half *)y, n, has_b, relu);
     } else return fail(ONE_ERR_UNSUPPORTED, "Add/Relu: dtype %d", dtype);
     count_launch();
     cudaError_t e = cudaGetLastError();
@@ -398,14 +406,14 @@ extern "C" int one_glue_gap_nhwc(const void *x, void *y, int dtype, int N, int H
     const int block = 128;
     const long long work = (long long)N * C;
     if (dtype == DT_F32 && C % 4 == 0 && aligned16(x) && aligned16(y))
-        k_gap_nhwc_vec<float><<<grid_for(work / 4, block), block, 0, st>>>((const float *)x, (float *)y, N, HW, C);
+        launch_k(k_gap_nhwc_vec<float>, grid_for(work / 4, block), block, 0, st, (const float *)x, (float *)y, N, HW, C);
     else if (dtype == DT_BF16 && C % 8 == 0 && aligned16(x) && aligned16(y))
-        k_gap_nhwc_vec<__nv_bfloat16><<<grid_for(work / 8, block), block, 0, st>>>((const __nv_bfloat16 *)x, (__nv_bfloat16 *)y, N, HW, C);
+        launch_k(k_gap_nhwc_vec<__nv_bfloat16>, grid_for(work / 8, block), block, 0, st, (const __nv_bfloat16 *)x, (__nv_bfloat16 *)y, N, HW, C);
     else if (dtype == DT_F16 && C % 8 == 0 && aligned16(x) && aligned16(y))
-        k_gap_nhwc_vec<__half><<<grid_for(work / 8, block), block, 0, st>>>((const __half *)x, (__half *)y, N, HW, C);
-    else if (dtype == DT_F32) k_gap_nhwc<float><<<grid_for(work, block), block, 0, st>>>((const float *)x, (float *)y, N, HW, C);
-    else if (dtype == DT_BF16) k_gap_nhwc<__nv_bfloat16><<<grid_for(work, block), block, 0, st>>>((const __nv_bfloat16 *)x, (__nv_bfloat16 *)y, N, HW, C);
-    else if (dtype == DT_F16) k_gap_nhwc<__half><<<grid_for(work, block), block, 0, st>>>((const __half *)x, (__half *)y, N, HW, C);
+        launch_k(k_gap_nhwc_vec<__half>, grid_for(work / 8, block), block, 0, st, (const __half *)x, (__half *)y, N, HW, C);
+    else if (dtype == DT_F32) launch_k(k_gap_nhwc<float>, grid_for(work, block), block, 0, st, (const float *)x, (float *)y, N, HW, C);
+    else if (dtype == DT_BF16) launch_k(k_gap_nhwc<__nv_bfloat16>, grid_for(work, block), block, 0, st, (const __nv_bfloat16 *)x, (__nv_bfloat16 *)y, N, HW, C);
+    else if (dtype == DT_F16) launch_k(k_gap_nhwc<__half>, grid_for(work, block), block, 0, st, (const __half *)x, (__half *)y, N, HW, C);
     else return fail(ONE_ERR_UNSUPPORTED, "GlobalAveragePool: dtype %d", dtype);
     count_launch();
     cudaError_t e = cudaGetLastError();
@@ -432,10 +440,10 @@ extern "C" int one_glue_cast(const void *x, void *y, int src_dtype, int dst_dtyp
     if (n <= 0) return ONE_OK;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const int block = 256;
-    if (src_dtype == DT_F32 && dst_dtype == DT_BF16) k_cast<float, __nv_bfloat16><<<grid_for(n, block), block, 0, st>>>((const float *)x, (__nv_bfloat16 *)y, n);
-    else if (src_dtype == DT_F32 && dst_dtype == DT_F16) k_cast<float, __half><<<grid_for(n, block), block, 0, st>>>((const float *)x, (__half *)y, n);
-    else if (src_dtype == DT_BF16 && dst_dtype == DT_F32) k_cast<__nv_bfloat16, float><<<grid_for(n, block), block, 0, st>>>((const __nv_bfloat16 *)x, (float *)y, n);
-    else if (src_dtype == DT_F16 && dst_dtype == DT_F32) k_cast<__half, float><<<grid_for(n, block), block, 0, st>>>((const __half *)x, (float *)y, n);
+    if (src_dtype == DT_F32 && dst_dtype == DT_BF16) launch_k(k_cast<float, __nv_bfloat16>, grid_for(n, block), block, 0, st, (const float *)x, (__nv_bfloat16 *)y, n);
+    else if (src_dtype == DT_F32 && dst_dtype == DT_F16) launch_k(k_cast<float, __half>, grid_for(n, block), block, 0, st, (const float *)x, (__half *)y, n);
+    else if (src_dtype == DT_BF16 && dst_dtype == DT_F32) launch_k(k_cast<__nv_bfloat16, float>, grid_for(n, block), block, 0, st, (const __nv_bfloat16 *)x, (float *)y, n);
+    else if (src_dtype == DT_F16 && dst_dtype == DT_F32) launch_k(k_cast<__half, float>, grid_for(n, block), block, 0, st, (const __half *)x, (float *)y, n);
     else return fail(ONE_ERR_UNSUPPORTED, "cast %d -> %d", src_dtype, dst_dtype);
     count_launch();
     cudaError_t e = cudaGetLastError();

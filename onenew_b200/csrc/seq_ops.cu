@@ -16,6 +16,7 @@
 //       applied as a multiplication by its reciprocal, device/x86/Div/div.c:104-118).
 #include "../../include/one_glue.h"
 #include "ctx.h"
+#include "launch.cuh"
 
 using namespace one;
 
@@ -48,6 +49,7 @@ template <int RV>   // float4 per lane kept in registers
 __global__ void k_layernorm(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ b,
                             float *__restrict__ y, long long rows, int D)
 {
+    pdl_entry(x, w, b);
     const int lane = threadIdx.x & 31;
     const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -93,6 +95,7 @@ __global__ void k_layernorm(const float *__restrict__ x, const float *__restrict
 __global__ void k_layernorm_any(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ b,
                                 float *__restrict__ y, long long rows, int D)
 {
+    pdl_entry(x, w, b);
     const int lane = threadIdx.x & 31;
     const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -125,6 +128,7 @@ __device__ __forceinline__ float gelu_lut(float v, const float *__restrict__ lut
 template <bool VEC>
 __global__ void k_gelu(const float *__restrict__ x, const float *__restrict__ lut, float *__restrict__ y, long long n)
 {
+    pdl_entry(x, lut);
     const long long stride = (long long)gridDim.x * blockDim.x;
     if (VEC) {
         const long long nv = n >> 2;
@@ -143,6 +147,7 @@ __global__ void k_gelu(const float *__restrict__ x, const float *__restrict__ lu
 template <int RV>
 __global__ void k_softmax(const float *__restrict__ x, float *__restrict__ y, long long rows, int D)
 {
+    pdl_entry(x);
     const int lane = threadIdx.x & 31;
     const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -175,6 +180,7 @@ __global__ void k_softmax(const float *__restrict__ x, float *__restrict__ y, lo
 }
 __global__ void k_softmax_any(const float *__restrict__ x, float *__restrict__ y, long long rows, int D)
 {
+    pdl_entry(x);
     const int lane = threadIdx.x & 31;
     const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -203,6 +209,7 @@ struct Dims6 {
 // Generic gather: consecutive threads write consecutive outputs.
 __global__ void k_transpose(const float *__restrict__ x, float *__restrict__ y, long long n, Dims6 d)
 {
+    pdl_entry(x);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         long long t = i, off = 0;
 #pragma unroll
@@ -220,6 +227,7 @@ __global__ void k_transpose(const float *__restrict__ x, float *__restrict__ y, 
 __global__ void k_transpose_tile(const float *__restrict__ x, float *__restrict__ y, Dims6 d, int A, int B,
                                  long long stride_b_in)
 {
+    pdl_entry(x);
     __shared__ float tile[32][33];
     long long z = blockIdx.z, off_in = 0;
 #pragma unroll
@@ -248,6 +256,7 @@ template <bool VEC>
 __global__ void k_copy_chunks(const float *__restrict__ x, float *__restrict__ y, long long reps, long long chunk,
                               long long x_reps, long long x_stride, long long y_stride)
 {
+    pdl_entry(x);
     const long long cw = VEC ? (chunk >> 2) : chunk;
     const long long total = reps * cw;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -274,6 +283,7 @@ template <int OP, bool VEC, bool SWAP>
 __global__ void k_binary_period(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ y, long long n,
                                 long long period)
 {
+    pdl_entry(a, b);
     const long long stride = (long long)gridDim.x * blockDim.x;
     if (VEC) {
         const long long nv = n >> 2, pv = period >> 2;
@@ -299,6 +309,7 @@ template <int OP>
 __global__ void k_binary_strided(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ y, long long n,
                                  Dims6 da, Dims6 db)
 {
+    pdl_entry(a, b);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         long long t = i, oa = 0, ob = 0;
 #pragma unroll
@@ -322,11 +333,11 @@ cudaError_t launch_binary_period(const float *a, const float *b, float *y, long 
     const int block = 256;
     const int grid = grid_for(vec ? n / 4 : n, block);
     if (vec) {
-        if (swap) k_binary_period<OP, true, true><<<grid, block, 0, st>>>(a, b, y, n, period);
-        else k_binary_period<OP, true, false><<<grid, block, 0, st>>>(a, b, y, n, period);
+        if (swap) launch_k(k_binary_period<OP, true, true>, grid, block, 0, st, a, b, y, n, period);
+        else launch_k(k_binary_period<OP, true, false>, grid, block, 0, st, a, b, y, n, period);
     } else {
-        if (swap) k_binary_period<OP, false, true><<<grid, block, 0, st>>>(a, b, y, n, period);
-        else k_binary_period<OP, false, false><<<grid, block, 0, st>>>(a, b, y, n, period);
+        if (swap) launch_k(k_binary_period<OP, false, true>, grid, block, 0, st, a, b, y, n, period);
+        else launch_k(k_binary_period<OP, false, false>, grid, block, 0, st, a, b, y, n, period);
     }
     return cudaGetLastError();
 }
@@ -341,9 +352,9 @@ extern "C" int one_glue_layernorm(const float *x, const float *w, const float *b
     const int block = 256;
     const int grid = grid_for(rows * 32, block);
     const bool vec = D % 4 == 0 && aligned16(x) && aligned16(y) && aligned16(w) && aligned16(b);
-    if (vec && D <= 256) k_layernorm<2><<<grid, block, 0, st>>>(x, w, b, y, rows, D);
-    else if (vec && D <= 1024) k_layernorm<8><<<grid, block, 0, st>>>(x, w, b, y, rows, D);
-    else k_layernorm_any<<<grid, block, 0, st>>>(x, w, b, y, rows, D);
+    if (vec && D <= 256) launch_k(k_layernorm<2>, grid, block, 0, st, x, w, b, y, rows, D);
+    else if (vec && D <= 1024) launch_k(k_layernorm<8>, grid, block, 0, st, x, w, b, y, rows, D);
+    else launch_k(k_layernorm_any, grid, block, 0, st, x, w, b, y, rows, D);
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ONE_OK : cuda_fail(e, "layernorm launch");
@@ -355,8 +366,8 @@ extern "C" int one_glue_gelu_lut(const float *x, const float *lut, float *y, lon
     if (n == 0) return ONE_OK;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const bool vec = n % 4 == 0 && aligned16(x) && aligned16(y);
-    if (vec) k_gelu<true><<<grid_for(n / 4, 256), 256, 0, st>>>(x, lut, y, n);
-    else k_gelu<false><<<grid_for(n, 256), 256, 0, st>>>(x, lut, y, n);
+    if (vec) launch_k(k_gelu<true>, grid_for(n / 4, 256), 256, 0, st, x, lut, y, n);
+    else launch_k(k_gelu<false>, grid_for(n, 256), 256, 0, st, x, lut, y, n);
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ONE_OK : cuda_fail(e, "gelu launch");
@@ -369,10 +380,10 @@ extern "C" int one_glue_softmax_rows(const float *x, float *y, long long rows, i
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const int block = 256;
     const int grid = grid_for(rows * 32, block);
-    if (D <= 64) k_softmax<2><<<grid, block, 0, st>>>(x, y, rows, D);
-    else if (D <= 256) k_softmax<8><<<grid, block, 0, st>>>(x, y, rows, D);
-    else if (D <= 1024) k_softmax<32><<<grid, block, 0, st>>>(x, y, rows, D);
-    else k_softmax_any<<<grid, block, 0, st>>>(x, y, rows, D);
+    if (D <= 64) launch_k(k_softmax<2>, grid, block, 0, st, x, y, rows, D);
+    else if (D <= 256) launch_k(k_softmax<8>, grid, block, 0, st, x, y, rows, D);
+    else if (D <= 1024) launch_k(k_softmax<32>, grid, block, 0, st, x, y, rows, D);
+    else launch_k(k_softmax_any, grid, block, 0, st, x, y, rows, D);
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ONE_OK : cuda_fail(e, "softmax launch");
@@ -403,9 +414,9 @@ extern "C" int one_glue_transpose(const float *x, float *y, int ndim, const int 
     // out[.., a, b] with the input contiguous along a (stride 1) and b a strided input dim
     if (d.stride[4] == 1 && d.shape[4] >= 8 && d.shape[5] >= 8 && outer <= 0x7fffffffLL / 2 && outer <= 65535) {
         dim3 grid((d.shape[5] + 31) / 32, (d.shape[4] + 31) / 32, (unsigned)outer), block(32, 8);
-        k_transpose_tile<<<grid, block, 0, st>>>(x, y, d, d.shape[4], d.shape[5], d.stride[5]);
+        launch_k(k_transpose_tile, grid, block, 0, st, x, y, d, d.shape[4], d.shape[5], d.stride[5]);
     } else {
-        k_transpose<<<grid_for(n, 256), 256, 0, st>>>(x, y, n, d);
+        launch_k(k_transpose, grid_for(n, 256), 256, 0, st, x, y, n, d);
     }
     count_launch();
     cudaError_t e = cudaGetLastError();
@@ -419,8 +430,8 @@ extern "C" int one_glue_copy_chunks(const float *x, float *y, long long reps, lo
     if (reps == 0 || chunk == 0) return ONE_OK;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const bool vec = chunk % 4 == 0 && x_stride % 4 == 0 && y_stride % 4 == 0 && aligned16(x) && aligned16(y);
-    if (vec) k_copy_chunks<true><<<grid_for(reps * (chunk / 4), 256), 256, 0, st>>>(x, y, reps, chunk, x_reps, x_stride, y_stride);
-    else k_copy_chunks<false><<<grid_for(reps * chunk, 256), 256, 0, st>>>(x, y, reps, chunk, x_reps, x_stride, y_stride);
+    if (vec) launch_k(k_copy_chunks<true>, grid_for(reps * (chunk / 4), 256), 256, 0, st, x, y, reps, chunk, x_reps, x_stride, y_stride);
+    else launch_k(k_copy_chunks<false>, grid_for(reps * chunk, 256), 256, 0, st, x, y, reps, chunk, x_reps, x_stride, y_stride);
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ONE_OK : cuda_fail(e, "copy_chunks launch");
@@ -481,10 +492,10 @@ extern "C" int one_glue_binary(int op, const float *a, const float *b, float *y,
         }
         const int grid = grid_for(n, 256);
         switch (op) {
-        case 0: k_binary_strided<0><<<grid, 256, 0, st>>>(a, b, y, n, da, db); break;
-        case 1: k_binary_strided<1><<<grid, 256, 0, st>>>(a, b, y, n, da, db); break;
-        case 2: k_binary_strided<2><<<grid, 256, 0, st>>>(a, b, y, n, da, db); break;
-        default: k_binary_strided<3><<<grid, 256, 0, st>>>(a, b, y, n, da, db); break;
+        case 0: launch_k(k_binary_strided<0>, grid, 256, 0, st, a, b, y, n, da, db); break;
+        case 1: launch_k(k_binary_strided<1>, grid, 256, 0, st, a, b, y, n, da, db); break;
+        case 2: launch_k(k_binary_strided<2>, grid, 256, 0, st, a, b, y, n, da, db); break;
+        default: launch_k(k_binary_strided<3>, grid, 256, 0, st, a, b, y, n, da, db); break;
         }
         e = cudaGetLastError();
     }
