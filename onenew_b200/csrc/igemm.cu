@@ -24,6 +24,7 @@
 #include "igemm.cuh"
 #include "sm100_prims.cuh"
 #include "act.cuh"
+#include "round_tf32.cuh"
 #include "ctx.h"
 #include "launch.cuh"
 
@@ -72,27 +73,6 @@ __host__ __device__ constexpr size_t smem_layout_bytes(int bn, bool pair = false
 }
 
 size_t igemm_smem_bytes(int bn, bool pair, int mh, int nw) { return smem_layout_bytes(bn, pair, mh, nw) + 1024; }
-
-// Round to the nearest tf32 (10 mantissa bits), ties away from zero, like cvt.rna.tf32.f32 -- but with
-// two integer instructions: the conversion instruction runs on the 16-lane special-function pipe and,
-// at one per output element, was a measurable share of the epilogue (that pipe 42 % busy on a 3x3
-// 64-channel layer).  Adding half an ulp to the magnitude bits and clearing the low 13 carries into the
-// exponent correctly.  Infinities and NaNs (exponent all ones) pass through untouched: the add would
-// carry a NaN's mantissa into the sign bit and turn it into -0.0, and cvt.rna keeps NaNs too.
-__device__ __forceinline__ float round_to_tf32(float v)
-{
-    const uint32_t u = __float_as_uint(v);
-    return ((u & 0x7f800000u) == 0x7f800000u) ? v : __uint_as_float((u + 0x1000u) & 0xffffe000u);
-}
-
-// Quantise for an int8 consumer: x * (1/scale), clamp to [-128, 127], roundf
-// (device/x86/Conv/conv.c:961-973).
-__device__ __forceinline__ int quant_s8(float v, float inv_scale)
-{
-    float t = __fmul_rn(v, inv_scale);
-    t = (t < -128.f) ? -128.f : (t > 127.f) ? 127.f : t;
-    return (int)roundf(t);
-}
 
 // A 32-row x 64-column patch of 16-bit values in shared memory, as the TMA store / load with a 128-byte
 // swizzle lays it out: 128-byte rows, 16-byte piece j of row r at j ^ (r & 7); lane = row; half h of the
@@ -830,6 +810,30 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                         patch = patch_alt;
                         patch_alt = t;
                     }
+                    continue;
+                }
+                if (p.nchw_hw) {
+                    uint32_t r[32];
+                    tmem_ld_32x32(taddr + c0, r);
+                    tmem_ld_wait();
+                    const int m = row0 + lane;
+                    if (m < p.M) {
+                        const int img = m / p.nchw_hw, nc = n0 + c0;
+                        float *o = reinterpret_cast<float *>(p.out) + ((long long)img * p.N + nc) * p.nchw_hw + (m - img * p.nchw_hw);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            if (nc + j >= p.N) break;
+                            const float b = p.bias ? __ldg(reinterpret_cast<const float *>(p.bias) + nc + j) : 0.f;
+                            float t;
+                            if constexpr (KIND == KIND_I8) t = __fmul_rn(__fadd_rn(__fmul_rn(__int2float_rn((int)r[j]), p.in_scale), b), __ldg(p.coeff + nc + j));
+                            else t = __fadd_rn(__uint_as_float(r[j]), b);
+                            if (act == 1) t = t > 0.f ? t : 0.f;
+                            else if (act == 3) t = silu_table(t, p.lut_smem ? slut : p.lut);
+                            else if (act != 0) t = apply_act(t, act, p.act_p0, p.act_p1, p.lut);
+                            o[(long long)j * p.nchw_hw] = t;
+                        }
+                    }
+                    __syncwarp();
                     continue;
                 }
                 // this lane's 4 columns and their per-column constants (issued before the TMEM load so

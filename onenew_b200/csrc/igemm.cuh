@@ -41,6 +41,8 @@ struct IgemmParams {
     int lut_smem;         // stage the table in shared memory (only without a residual; 16-byte aligned table)
     const void *residual; // optional [M][ldo], same element type as out; added before res_relu
     int res_relu;         // relu after the residual add
+    int nchw_hw;          // > 0: out is fp32 [M / hw][N][hw], the reference layout of a convolution's output (no residual,
+                          // out_q or tma_store): lane = pixel in the accumulator, so plain stores are whole lines
     int round_tf32;       // round f32 outputs to tf32 (nearest) so a tf32 consumer sees exact values
     int ab_f16;           // 16-bit kind: the operands are fp16, not bf16
     int res_mma;          // 16-bit kinds, plain tiles, 128-byte slabs: the residual is added by the tensor core -- the

@@ -26,6 +26,8 @@
 #include "ctx.h"
 #include "glue.cuh"
 #include "igemm.cuh"
+#include "igemm_unit.cuh"
+#include <stdlib.h>
 #include "sm100_prims.cuh"
 
 using namespace one;
@@ -39,6 +41,7 @@ static std::atomic<int> g_half_tiles{1};  // tile codes 2xxx (two 128-row halves
 static std::atomic<int> g_wide_epi{1};    // tile codes 4xxx (twelve epilogue warps) are accepted
 thread_local int t_pairing = 1;      // width pairing of narrow multi-tap convolutions (see pair_geometry)
 thread_local int t_last_split = 1;   // K ranges the last contraction enqueued by this thread was cut into
+thread_local int t_last_unit = 0;    // whether it took the unit kernel
 thread_local int t_split_k = 0;   // 0: the library's choice, 1: never split, n > 1: force n ranges (clamped to the K blocks)
 
 struct ConvGeom {
@@ -58,6 +61,7 @@ struct ConvPlan {
     int cta2;                 // launch as pairs of CTAs sharing 256-row tiles (tile codes 1xxx)
     int mh;                   // 128-row halves per CTA tile: 1, or 2 (tile codes 2xxx)
     int nw;                   // epilogue warps: 8, or 12 (tile codes 4xxx)
+    int auto_tile;            // the tile is the library's choice (a launch of about one wave may then take the unit kernel)
     // PATH_S2D: the stride-2 conv re-expressed as a stride-1 conv over the space-to-depth image;
     // bw = columns carried per position (2, or 4: neighbouring positions overlap and one filter
     // position covers 4 taps along w, placed dil_w = bw / 2 positions apart)
@@ -163,6 +167,21 @@ int run_split(one_ctx *ctx, int kind, int bn, const CUtensorMap &tmA, const CUte
     if (ce != cudaSuccess) return cuda_fail(ce, "igemm launch (split-K)");
     if ((ce = launch_splitk_reduce(r, stream)) != cudaSuccess) return cuda_fail(ce, "split-K reduce launch");
     return ONE_OK;
+}
+
+// The unit kernel (igemm_unit.cu): chosen when the library picks the tile and the split, and the launch has at most
+// UNIT_MAX_TILES tiles of 128 x 64.  Returns the CTAs per tile along K (1, 2, 4 or 8; 0: take the persistent kernel).
+int choose_unit(int auto_tile, long long M, int N, int batch, int num_kb)
+{
+    if (!auto_tile || t_split_k != 0) return 0;
+    const long long tiles = ((M + 127) / 128) * ((N + UNIT_BN - 1) / UNIT_BN) * (batch > 0 ? batch : 1);
+    static const long long lim = getenv("UNIT_TILES") ? atoll(getenv("UNIT_TILES")) : 148;
+    static const long long fill = getenv("UNIT_FILL") ? atoll(getenv("UNIT_FILL")) : 148;
+    static const int minkb = getenv("UNIT_MINKB") ? atoi(getenv("UNIT_MINKB")) : 2;
+    if (tiles > lim) return 0;
+    int s = 1;
+    while (s < 8 && tiles * s * 2 <= fill && num_kb >= s * 2 * minkb) s *= 2;
+    return s;
 }
 
 // Whether the final output of `p` can be produced by the split-K reduce kernel (float path, 16-byte rows).
@@ -310,6 +329,7 @@ void plan_conv(const ConvGeom &g, int kind, ConvPlan *p, bool x_nchw_f32)
     p->cta2 = tile_cta2(code) ? 1 : 0;
     p->mh = tile_mh(code);
     p->nw = tile_nw(code);
+    p->auto_tile = !valid_tile(t_tile_n);
 }
 
 // Width pairing.  A 128 x 64 tensor-core instruction takes as long as a 128 x 128 one, so a convolution
@@ -376,6 +396,8 @@ struct ConvIO {
     int8_t *out_q;
     float q_inv_scale;
     float x_inv_scale;    // int8 + x_nchw_f32 explicit path: quantise while packing
+    int y_nchw;           // y is fp32 in the reference layout
+    int w_const;          // w holds weights prepared before this call
 };
 
 // Store map for the epilogue's TMA path; *use is set to 1 when the output qualifies (no int8 copy, N a
@@ -491,7 +513,21 @@ int run_conv(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &
     p.lut_smem = p.act == SILU && p.lut && !p.residual && (reinterpret_cast<uintptr_t>(p.lut) & 15) == 0;
     p.out_q = io.out_q; p.q_inv_scale = io.q_inv_scale;
     p.status = ctx->status_dev;
-    if (!pl.cta2 && pl.mh == 1 && pl.nw == 8 && split_eligible(pl.kind, p)) {
+    UnitParams u;
+    memset(&u, 0, sizeof(u));
+    u.b_const = io.w_const; u.nchw_hw = io.y_nchw ? g.OH * g.OW : 0;
+    if ((u.splits = choose_unit(pl.auto_tile, M, g.OC, 0, pl.num_kb)) && unit_epilogue(pl.kind, p, u) >= 0) {
+        CUtensorMap tmU;
+        rc = make_tmap_tiled(&tmU, kind_tm(pl.kind), io.w, pl.w_pitch, g.OC, 0, (uint64_t)pl.w_pitch * pl.es, 0, pl.slab_elems, UNIT_BN, pl.slab_bytes);
+        if (rc != ONE_OK) return rc;
+        t_last_split = u.splits;
+        t_last_unit = 1;
+        cudaError_t ce = launch_unit(pl.kind, tmA, tmU, p, u, stream);
+        return ce == cudaSuccess ? ONE_OK : cuda_fail(ce, "unit launch");
+    }
+    t_last_unit = 0;
+    if (io.y_nchw) p.nchw_hw = g.OH * g.OW;
+    if (!io.y_nchw && !pl.cta2 && pl.mh == 1 && pl.nw == 8 && split_eligible(pl.kind, p)) {
         int per = 0;
         const int splits = choose_split(ctx, M, g.OC, pl.bn, pl.num_kb, &per);
         if (splits > 1 && (rc = run_split(ctx, pl.kind, pl.bn, tmA, tmB, p, splits, per, stream)) != 1) {
@@ -516,7 +552,7 @@ int run_conv(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &
         p.act = p.res_relu ? RELU : 0;
         p.res_relu = 0;
     }
-    if ((rc = make_store_map(pl.kind, &tmC, &tmR, &p.tma_store, p.out, p.out_mode, M, g.OC, p.ldo, 0, 0, p.residual, p.out_q)) != ONE_OK) return rc;
+    if (!io.y_nchw && (rc = make_store_map(pl.kind, &tmC, &tmR, &p.tma_store, p.out, p.out_mode, M, g.OC, p.ldo, 0, 0, p.residual, p.out_q)) != ONE_OK) return rc;
     if (!vec_constants_ok(p)) p.tma_store = 0;
     if (res_mma) {
         const int f = pl.kind == KIND_F16 ? 1 : 0;
@@ -570,7 +606,7 @@ struct GemmEpi {
 // Plain GEMM D[M,N] = A[M,K] * B[N,K]^T (+bias, +activation, +residual), optionally batched.
 int run_gemm(one_ctx *ctx, int kind, const void *A, int a_pitch, const void *B, int b_pitch, long long M, int N,
              int K, int batch, long long a_bstride, long long b_bstride, void *out, long long ldo,
-             long long out_bstride, int out_mode, const float *bias, const CUtensorMap *tmB_cached, int bn,
+             long long out_bstride, int out_mode, const float *bias, const CUtensorMap *tmB_cached, int bn, int auto_tile,
              cudaStream_t stream, const GemmEpi *epi = nullptr)
 {
     if (M > 0x7fffffffLL) return fail(ONE_ERR_BAD_SHAPE, "GEMM: M too large");
@@ -584,12 +620,6 @@ int run_gemm(one_ctx *ctx, int kind, const void *A, int a_pitch, const void *B, 
     int rc = make_tmap_tiled(&tmA, kind_tm(kind), A, K, M, batch, (uint64_t)a_pitch * es, (uint64_t)a_bstride * es,
                              slab_elems, 128, slab_bytes);
     if (rc != ONE_OK) return rc;
-    if (tmB_cached) tmB = *tmB_cached;
-    else {
-        rc = make_tmap_tiled(&tmB, kind_tm(kind), B, K, N, batch, (uint64_t)b_pitch * es, (uint64_t)b_bstride * es,
-                             slab_elems, cta2 ? bn / 2 : bn, slab_bytes);
-        if (rc != ONE_OK) return rc;
-    }
     IgemmParams p;
     memset(&p, 0, sizeof(p));
     p.M = (int)M; p.N = N; p.num_kb = (int)(((long long)K * es + slab_bytes - 1) / slab_bytes);
@@ -600,6 +630,21 @@ int run_gemm(one_ctx *ctx, int kind, const void *A, int a_pitch, const void *B, 
     if (epi) { p.act = epi->act; p.lut = epi->lut; p.residual = epi->residual; }
     p.lut_smem = p.act == SILU && p.lut && !p.residual && (reinterpret_cast<uintptr_t>(p.lut) & 15) == 0;
     p.status = ctx->status_dev;
+    UnitParams u;
+    memset(&u, 0, sizeof(u));
+    u.b_const = tmB_cached != nullptr;
+    t_last_unit = (u.splits = choose_unit(auto_tile, M, N, batch, p.num_kb)) && unit_epilogue(kind, p, u) >= 0;
+    if (tmB_cached && !t_last_unit) tmB = *tmB_cached;
+    else {
+        rc = make_tmap_tiled(&tmB, kind_tm(kind), B, K, N, batch, (uint64_t)b_pitch * es, (uint64_t)b_bstride * es,
+                             slab_elems, t_last_unit ? UNIT_BN : (cta2 ? bn / 2 : bn), slab_bytes);
+        if (rc != ONE_OK) return rc;
+    }
+    if (t_last_unit) {
+        t_last_split = u.splits;
+        cudaError_t ce = launch_unit(kind, tmA, tmB, p, u, stream);
+        return ce == cudaSuccess ? ONE_OK : cuda_fail(ce, "unit launch");
+    }
     if (!cta2 && mh == 1 && nw == 8 && split_eligible(kind, p)) {
         int per = 0;
         const int splits = choose_split(ctx, M, N, bn, p.num_kb, &per);
@@ -655,7 +700,7 @@ size_t conv_eval_scratch(const ConvGeom &g, const ConvEpi &e, const ConvPlan &pl
     if (pl.path == PATH_EXPLICIT || pl.path == PATH_PATCH) need += up256((size_t)M * pl.w_pitch * pl.es);
     else if (pl.path == PATH_S2D) need += up256((size_t)g.N * pl.Hs * pl.Ws * pl.Cp * pl.es);
     else need += up256((size_t)g.N * g.H * g.W * g.C * pl.es);
-    need += up256((size_t)g.OC * pl.w_pitch * pl.es) + up256((size_t)M * g.OC * 4);
+    need += up256((size_t)g.OC * pl.w_pitch * pl.es);
     if (e.int8) need += 2 * up256((size_t)g.OC * 4);
     return need;
 }
@@ -784,7 +829,6 @@ extern "C" int one_cuda_conv_eval(BUFFER_INFO_S *params, BUFFER_INFO_S *inputs, 
     const int kind = e.int8 ? KIND_I8 : kind_of_prec(t_eval_prec);
     ConvPlan pl;
     plan_conv(g, kind, &pl, true);
-    const long long M = (long long)g.N * g.OH * g.OW;
     if (conv_eval_scratch(g, e, pl) > ctx->ws_bytes)   // refused before anything is launched
         return fail(ONE_ERR_NOMEM, "Conv: this shape needs %zu bytes of scratch, the workspace holds %zu", conv_eval_scratch(g, e, pl), ctx->ws_bytes);
     const float inv_scale = e.int8 ? 1.0f / e.in_scale : 1.f;   // conv.c:943
@@ -803,8 +847,7 @@ extern "C" int one_cuda_conv_eval(BUFFER_INFO_S *params, BUFFER_INFO_S *inputs, 
         io.x = xh;
     }
     void *wp = ws_alloc(ctx, (size_t)g.OC * pl.w_pitch * pl.es);
-    float *yh = reinterpret_cast<float *>(ws_alloc(ctx, (size_t)M * g.OC * 4));
-    if (!wp || !yh) return fail(ONE_ERR_NOMEM, "Conv: workspace too small (weights / NHWC output)");
+    if (!wp) return fail(ONE_ERR_NOMEM, "Conv: workspace too small (weights)");
     ce = pack_weights_for(g, pl, reinterpret_cast<const void *>(inputs[1].addr), wp, e.int8, st);
     if (ce != cudaSuccess) return cuda_fail(ce, "pack_conv_weight");
     io.w = wp;
@@ -825,11 +868,10 @@ extern "C" int one_cuda_conv_eval(BUFFER_INFO_S *params, BUFFER_INFO_S *inputs, 
             return cuda_fail(ce, "coefficient upload");
         io.coeff = cd;
     }
-    io.y = yh;
+    io.y = reinterpret_cast<void *>(outputs[0].addr);   // the epilogue writes the reference layout itself
+    io.y_nchw = 1;
     io.out_mode = OUT_F32;
     if ((rc = run_conv(ctx, g, e, pl, io, nullptr, st)) != ONE_OK) return rc;
-    ce = nhwc_to_nchw(yh, reinterpret_cast<float *>(outputs[0].addr), g.N, g.OC, g.OH * g.OW, DT_F32, st);
-    if (ce != cudaSuccess) return cuda_fail(ce, "nhwc_to_nchw");
     return finish_sync(ctx, st);
 }
 
@@ -860,7 +902,7 @@ extern "C" int one_cuda_gemm_eval(BUFFER_INFO_S *params, BUFFER_INFO_S *inputs, 
     if (ce == cudaSuccess) ce = pack_rows(reinterpret_cast<const float *>(inputs[1].addr), wp, N, K, Kp, kind_dt(kind), st);
     if (ce != cudaSuccess) return cuda_fail(ce, "pack_rows");
     rc = run_gemm(ctx, kind, ap, Kp, wp, Kp, M, N, K, 0, 0, 0, reinterpret_cast<void *>(outputs[0].addr), N, 0, OUT_F32,
-                  reinterpret_cast<const float *>(inputs[2].addr), nullptr, pick_bn(N, M), st);
+                  reinterpret_cast<const float *>(inputs[2].addr), nullptr, pick_bn(N, M), !valid_tile(t_tile_n), st);
     if (rc != ONE_OK) return rc;
     return finish_sync(ctx, st);
 }
@@ -899,10 +941,10 @@ static int matmul_enqueue(one_ctx *ctx, int kind, BUFFER_INFO_S *params, BUFFER_
     if (ce != cudaSuccess) return cuda_fail(ce, "MatMul operand packing");
     void *out = reinterpret_cast<void *>(outputs[0].addr);
     if (s.b_shared)   // every batch shares B: one GEMM over batch*M rows
-        rc = run_gemm(ctx, kind, A, a_pitch, bp, Kp, rowsA, s.N, s.K, 0, 0, 0, out, s.N, 0, OUT_F32, nullptr, nullptr, pick_bn(s.N, rowsA), st);
+        rc = run_gemm(ctx, kind, A, a_pitch, bp, Kp, rowsA, s.N, s.K, 0, 0, 0, out, s.N, 0, OUT_F32, nullptr, nullptr, pick_bn(s.N, rowsA), !valid_tile(t_tile_n), st);
     else
         rc = run_gemm(ctx, kind, A, a_pitch, bp, Kp, s.M, s.N, s.K, s.batch, (long long)s.M * a_pitch, (long long)s.N * Kp, out, s.N,
-                      (long long)s.M * s.N, OUT_F32, nullptr, nullptr, pick_bn(s.N, (long long)s.M * s.batch), st);
+                      (long long)s.M * s.N, OUT_F32, nullptr, nullptr, pick_bn(s.N, (long long)s.M * s.batch), !valid_tile(t_tile_n), st);
     if (flops) *flops = 2.0 * (double)rowsA * s.N * s.K;
     if (bytes) *bytes = ((double)rowsA * s.K + (double)nb * s.K * s.N + (double)rowsA * s.N) * 4.0;
     return rc;
@@ -946,7 +988,7 @@ struct one_packed {
     ConvEpi e;
     ConvPlan pl;
     // Gemm / MatMul
-    int M, K, N, Kp, b_shared, bn;
+    int M, K, N, Kp, b_shared, bn, auto_tile;
     // device-resident constants
     void *w = nullptr;
     void *bias = nullptr;
@@ -1106,6 +1148,7 @@ static int prepare_gemm(one_packed *op, bool is_gemm, BUFFER_INFO_S *params, BUF
         long long rows = 1;
         for (int i = 0; i < a0->dim_num_of_shapes - 1 && i < SHAPE_LEN; ++i) rows *= a0->shapes[i];
         op->bn = pick_bn(op->N, rows);
+        op->auto_tile = !valid_tile(t_tile_n);
     }
     if ((rc = upload(tmp, reinterpret_cast<const void *>(inputs[1].addr), (size_t)op->K * op->N * 4)) != ONE_OK) return rc;
     cudaError_t ce = cudaMalloc(&op->w, (size_t)op->N * op->Kp * es);
@@ -1191,6 +1234,7 @@ extern "C" int one_cuda_eval_async(one_ctx *ctx, one_packed *op, BUFFER_INFO_S *
         ConvIO io;
         memset(&io, 0, sizeof(io));
         io.w = op->w; io.bias = op->bias; io.coeff = op->coeff; io.lut = op->lut;
+        io.w_const = 1;
         const float inv_scale = op->e.int8 ? 1.0f / op->e.in_scale : 1.f;
         cudaError_t ce;
         int rc;
@@ -1206,12 +1250,8 @@ extern "C" int one_cuda_eval_async(one_ctx *ctx, one_packed *op, BUFFER_INFO_S *
                     return cuda_fail(ce, "nchw_to_nhwc");
                 io.x = xh;
             }
-            float *yh = reinterpret_cast<float *>(ws_alloc(ctx, (size_t)M * g.OC * 4));
-            if (!yh) return fail(ONE_ERR_NOMEM, "Conv: workspace too small for the NHWC output");
-            io.y = yh; io.out_mode = OUT_F32;
+            io.y = reinterpret_cast<void *>(outputs[0].addr); io.y_nchw = 1; io.out_mode = OUT_F32;
             if ((rc = run_conv(ctx, g, op->e, op->pl, io, &op->tmB, st)) != ONE_OK) return rc;
-            if ((ce = nhwc_to_nchw(yh, reinterpret_cast<float *>(outputs[0].addr), g.N, g.OC, g.OH * g.OW, DT_F32, st)) != cudaSuccess)
-                return cuda_fail(ce, "nhwc_to_nchw");
         } else {
             // device-resident NHWC activations
             if (op->flags & ONE_IN_NCHW_F32) {
@@ -1254,7 +1294,7 @@ extern "C" int one_cuda_eval_async(one_ctx *ctx, one_packed *op, BUFFER_INFO_S *
         }
         snprintf(op->detail, sizeof(op->detail), "M=%lld N=%d K=%d %dx%d/%d C=%d@%dx%d %s tile=128x%d split=%d%s%s", M, g.OC, g.C * g.KH * g.KW, g.KH, g.KW,
                  g.sh, g.C, g.H, g.W, kind_name(op->kind), op->pl.bn, t_last_split,
-                 op->paired ? " paired" : "", op->pl.cta2 ? " 2cta" : (op->pl.mh == 2 ? " 2half" : (op->pl.nw == 12 ? " 12w" : "")));
+                 op->paired ? " paired" : "", t_last_unit ? " unit" : op->pl.cta2 ? " 2cta" : (op->pl.mh == 2 ? " 2half" : (op->pl.nw == 12 ? " 12w" : "")));
         op->flops = 2.0 * (double)M * g.OC * g.C * g.KH * g.KW;   // host/ops/conv.h:159-176
         const double aes = (op->flags & ONE_IN_S8) ? 1.0 : (op->e.int8 ? 4.0 : (nhwc && bf16 ? 2.0 : 4.0));
         const double yes = outputs[0].addr ? ((nhwc && ((bf16 && !(op->flags & ONE_OUT_F32)) || (op->flags & ONE_OUT_BF16))) ? 2.0 : 4.0) : 0.0;
@@ -1295,10 +1335,10 @@ extern "C" int one_cuda_eval_async(one_ctx *ctx, one_packed *op, BUFFER_INFO_S *
     }
     int rc = run_gemm(ctx, op->kind, A, a_pitch, op->w, op->Kp, rows, op->N, op->K, 0, 0, 0,
                       reinterpret_cast<void *>(outputs[0].addr), op->N, 0, out_mode, reinterpret_cast<const float *>(op->bias),
-                      &op->tmB, op->bn, st, &epi);
+                      &op->tmB, op->bn, op->auto_tile, st, &epi);
     if (rc != ONE_OK) return rc;
     snprintf(op->detail, sizeof(op->detail), "M=%lld N=%d K=%d %s tile=128x%d split=%d%s", rows, op->N, op->K, kind_name(op->kind), tile_bn(op->bn),
-             t_last_split, tile_cta2(op->bn) ? " 2cta" : (tile_mh(op->bn) == 2 ? " 2half" : (tile_nw(op->bn) == 12 ? " 12w" : "")));
+             t_last_split, t_last_unit ? " unit" : tile_cta2(op->bn) ? " 2cta" : (tile_mh(op->bn) == 2 ? " 2half" : (tile_nw(op->bn) == 12 ? " 12w" : "")));
     op->flops = 2.0 * (double)rows * op->N * op->K;
     op->bytes = (double)rows * op->K * (a_native ? es : 4) + (double)op->N * op->K * es +
                 (double)rows * op->N * (out_is_16(out_mode) ? 2 : 4) * (epi.residual ? 2 : 1);
@@ -1383,7 +1423,6 @@ extern "C" int one_cuda_conv_eval_static(BUFFER_INFO_S *params, BUFFER_INFO_S *i
     const int kind = e.int8 ? KIND_I8 : kind_of_prec(t_eval_prec);
     ConvPlan pl;
     plan_conv(g, kind, &pl, true);
-    const long long M = (long long)g.N * g.OH * g.OW;
     // everything this call will carve out of the array, checked before anything is launched
     const size_t need = conv_eval_scratch(g, e, pl);
     if (need > ctx->ws_bytes)
@@ -1406,8 +1445,7 @@ extern "C" int one_cuda_conv_eval_static(BUFFER_INFO_S *params, BUFFER_INFO_S *i
         io.x = xh;
     }
     void *wp = ws_alloc(ctx, (size_t)g.OC * pl.w_pitch * pl.es);
-    float *yh = reinterpret_cast<float *>(ws_alloc(ctx, (size_t)M * g.OC * 4));
-    if (!wp || !yh) return fail(ONE_ERR_NOMEM, "Conv (static scratch): weights / NHWC output do not fit");
+    if (!wp) return fail(ONE_ERR_NOMEM, "Conv (static scratch): weights do not fit");
     if ((ce = pack_weights_for(g, pl, reinterpret_cast<const void *>(inputs[1].addr), wp, e.int8, st)) != cudaSuccess)
         return cuda_fail(ce, "pack_conv_weight");
     io.w = wp;
@@ -1427,10 +1465,9 @@ extern "C" int one_cuda_conv_eval_static(BUFFER_INFO_S *params, BUFFER_INFO_S *i
         io.coeff = cd;
     }
     io.lut = reinterpret_cast<const float *>(inputs[BUF_MAXNUM - 1].addr);
-    io.y = yh;
+    io.y = reinterpret_cast<void *>(outputs[0].addr);
+    io.y_nchw = 1;
     io.out_mode = OUT_F32;
     if ((rc = run_conv(ctx, g, e, pl, io, nullptr, st)) != ONE_OK) return rc;
-    if ((ce = nhwc_to_nchw(yh, reinterpret_cast<float *>(outputs[0].addr), g.N, g.OC, g.OH * g.OW, DT_F32, st)) != cudaSuccess)
-        return cuda_fail(ce, "nhwc_to_nchw");
     return finish_sync(ctx, st);   // waits for the stream; `coeff` above stays alive until then
 }
