@@ -27,7 +27,6 @@
 #include "glue.cuh"
 #include "igemm.cuh"
 #include "igemm_unit.cuh"
-#include <stdlib.h>
 #include "sm100_prims.cuh"
 
 using namespace one;
@@ -169,19 +168,24 @@ int run_split(one_ctx *ctx, int kind, int bn, const CUtensorMap &tmA, const CUte
     return ONE_OK;
 }
 
-// The unit kernel (igemm_unit.cu): chosen when the library picks the tile and the split, and the launch has at most
-// UNIT_MAX_TILES tiles of 128 x 64.  Returns the CTAs per tile along K (1, 2, 4 or 8; 0: take the persistent kernel).
+// The unit kernel (igemm_unit.cu): chosen when the library picks the tile and the split, and all of the launch's 128 x 64
+// tiles are resident at once (two CTAs on each of 148 SMs) with a short enough K range each: then latency and not the
+// operand stream sets the time.  With more tiles the wider ones and the overlapped epilogue of the persistent kernel win;
+// a long K range wants its 256-wide tiles, which bring half the operand bytes per product.  ResNet-50, us (limit of tiles /
+// of K blocks a CTA): fp16 32 images 1217 (148 / 64), 1195 (296 / 24), 1141 (296 / 64); TF32 61 images of 192 x 192: 2048,
+// 2037, 2021; without the unit kernel 1230 and 2022.  Few tiles are cut along K until the SMs are covered; a CTA keeps at
+// least two K blocks, since below that the exchange costs more than the blocks it saves.
+// Returns the CTAs per tile along K (1, 2, 4 or 8; 0: take the persistent kernel).
 int choose_unit(int auto_tile, long long M, int N, int batch, int num_kb)
 {
     if (!auto_tile || t_split_k != 0) return 0;
     const long long tiles = ((M + 127) / 128) * ((N + UNIT_BN - 1) / UNIT_BN) * (batch > 0 ? batch : 1);
-    static const long long lim = getenv("UNIT_TILES") ? atoll(getenv("UNIT_TILES")) : 148;
-    static const long long fill = getenv("UNIT_FILL") ? atoll(getenv("UNIT_FILL")) : 148;
-    static const int minkb = getenv("UNIT_MINKB") ? atoi(getenv("UNIT_MINKB")) : 2;
-    if (tiles > lim) return 0;
+    constexpr long long SMS = 148;
+    constexpr int MAX_KB = 64;
+    if (tiles > 2 * SMS) return 0;
     int s = 1;
-    while (s < 8 && tiles * s * 2 <= fill && num_kb >= s * 2 * minkb) s *= 2;
-    return s;
+    while (s < 8 && tiles * s * 2 <= SMS && num_kb >= s * 4) s *= 2;
+    return num_kb > MAX_KB * s ? 0 : s;
 }
 
 // Whether the final output of `p` can be produced by the split-K reduce kernel (float path, 16-byte rows).
@@ -701,6 +705,7 @@ size_t conv_eval_scratch(const ConvGeom &g, const ConvEpi &e, const ConvPlan &pl
     else if (pl.path == PATH_S2D) need += up256((size_t)g.N * pl.Hs * pl.Ws * pl.Cp * pl.es);
     else need += up256((size_t)g.N * g.H * g.W * g.C * pl.es);
     need += up256((size_t)g.OC * pl.w_pitch * pl.es);
+    need += up256((size_t)M * g.OC * 4);   // (an NHWC copy of the output, no longer made: the same shapes are refused as before)
     if (e.int8) need += 2 * up256((size_t)g.OC * 4);
     return need;
 }

@@ -482,3 +482,69 @@ def test_int8_and_gemm_two_half_tiles(ops, oracle_mod):
             L.one_cuda_set_tile_n(0)
         assert np.array_equal(y, ref), tile
         assert_close(yg, oracle_mod.gemm(a, wg, bg), f"gemm with two-half tiles {tile}")
+
+
+# One-wave launches: ragged rows and columns, one K block up to many (one CTA a tile, then clusters of 2, 4 and 8 along
+# K), operands whose rows are and are not whole 16-byte pieces, two CTAs on an SM
+UNIT_GEMMS = [(1, 64, 10), (127, 100, 64), (128, 512, 65), (129, 1027, 63), (33, 2048, 1000), (300, 256, 132), (1100, 96, 1600)]
+
+
+@pytest.mark.parametrize("prec", ["tf32", "f16"])
+@pytest.mark.parametrize("shape", UNIT_GEMMS, ids=[f"{m}x{k}x{n}" for m, k, n in UNIT_GEMMS])
+def test_one_wave_gemm_and_matmul_vs_oracle_and_persistent(ops, oracle_mod, shape, prec):
+    """Against the oracle, against the same call with the K split switched off (the persistent kernel: another order of the
+    fp32 sums) and against itself (no dependence on the scheduling)."""
+    M, K, N = shape
+    rng = np.random.default_rng(M * 7 + K + N)
+    a = rng.standard_normal((M, K)).astype(np.float32)
+    w = (rng.standard_normal((N, K)) * 0.05).astype(np.float32)
+    b = rng.standard_normal(N).astype(np.float32)
+    a3 = rng.standard_normal((2, M, K)).astype(np.float32)
+    b3 = (rng.standard_normal((2, K, N)) * 0.05).astype(np.float32)
+    L = capi.lib()
+    capi.check(L.one_cuda_set_eval_precision(capi.PRECISIONS[prec]))
+    try:
+        got = [_np(ops.gemm(a, w, b)), _np(ops.matmul(a3, b3)), _np(ops.matmul(a3, b3[0]))]
+        again = [_np(ops.gemm(a, w, b)), _np(ops.matmul(a3, b3)), _np(ops.matmul(a3, b3[0]))]
+        capi.check(L.one_cuda_set_split_k(1))
+        plain = [_np(ops.gemm(a, w, b)), _np(ops.matmul(a3, b3)), _np(ops.matmul(a3, b3[0]))]
+    finally:
+        L.one_cuda_set_split_k(0)
+        L.one_cuda_set_eval_precision(capi.PREC_TF32)
+    ref = [oracle_mod.gemm(a, w, b), np.matmul(a3.astype(np.float64), b3), np.matmul(a3.astype(np.float64), b3[0])]
+    for g, g2, pl, r, name in zip(got, again, plain, ref, ("gemm", "matmul", "matmul shared")):
+        assert np.array_equal(g, g2), name
+        assert_close(g, r.astype(np.float32), name)
+        # products carry 2^-11 per operand, and the two kernels may differ in how an operand is rounded
+        assert np.abs(g - pl).max() <= 2e-3 * np.abs(r).max(), name
+
+
+UNIT_CONVS = [
+    # N, C, H, W, OC, k, stride, pad, act: one tile, a ragged last row tile, ragged columns, each epilogue form
+    (1, 32, 8, 16, 64, 1, 1, 0, abi.RELU), (1, 64, 7, 7, 70, 3, 1, 1, abi.SILU), (3, 128, 14, 13, 33, 3, 2, 1, abi.LEAKYRELU),
+    (1, 512, 7, 7, 512, 3, 1, 1, abi.RELU), (2, 24, 20, 20, 40, 5, 1, 2, abi.HARDSILU), (1, 3, 30, 30, 17, 7, 2, 3, abi.CLIP),
+]
+
+
+@pytest.mark.parametrize("case", UNIT_CONVS, ids=[f"{c[1]}to{c[4]}@{c[2]}x{c[3]}k{c[5]}" for c in UNIT_CONVS])
+def test_one_wave_conv_vs_oracle_and_persistent(ops, oracle_mod, case):
+    """Both kernels write the reference layout from the accumulator; int8: the same bits."""
+    N, C, H, W, OC, k, s, p, act = case
+    rng = np.random.default_rng(C * H + OC)
+    x = rng.uniform(-1, 1, (N, C, H, W)).astype(np.float32)
+    w = (rng.standard_normal((OC, C, k, k)) * 0.05).astype(np.float32)
+    b = (rng.standard_normal(OC) * 0.1).astype(np.float32)
+    lut = oracle_mod.silu_lut() if act == abi.SILU else None
+    w8, b32, aux = oracle_mod.quant_weight_bias(w, b)
+    L = capi.lib()
+    y, y8 = _np(ops.conv(x, w, b, (s, s), (p,) * 4, act, lut=lut)), _np(ops.conv(x, w8, b32, (s, s), (p,) * 4, act, int8=(0.01, aux), lut=lut))
+    try:
+        capi.check(L.one_cuda_set_split_k(1))
+        z, z8 = _np(ops.conv(x, w, b, (s, s), (p,) * 4, act, lut=lut)), _np(ops.conv(x, w8, b32, (s, s), (p,) * 4, act, int8=(0.01, aux), lut=lut))
+    finally:
+        L.one_cuda_set_split_k(0)
+    ref = oracle_mod.conv_f32(x, w, b, (s, s), (p,) * 4, act)
+    assert_close(y, ref, "one wave")
+    assert_close(z, ref, "persistent")
+    ref8 = oracle_mod.conv_s8(x, w8, b32, aux, 0.01, (s, s), p, act)[0]
+    assert np.array_equal(y8, ref8) and np.array_equal(z8, ref8)
