@@ -38,6 +38,7 @@ struct IgemmParams {
     int act;              // ACT_TYPE_E
     float act_p0, act_p1; // clip min/max | leaky alpha | hard-sigmoid alpha, beta
     const float *lut;     // SiLU / Gelu table (8192 entries)
+    int q_table;          // int8: no NaN can come out of the de-quantisation (finite coefficients, a scale below 2^90)
     int lut_smem;         // stage the table in shared memory (only without a residual; 16-byte aligned table)
     const void *residual; // optional [M][ldo], same element type as out; added before res_relu
     int res_relu;         // relu after the residual add

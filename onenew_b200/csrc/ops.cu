@@ -18,7 +18,9 @@
 // a tensor of another shape; equal strides, the only case the reference's models use, are unaffected.
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include <vector>
 
@@ -399,6 +401,7 @@ struct ConvIO {
     int round_tf32;
     int8_t *out_q;
     float q_inv_scale;
+    int coeff_finite;     // every int8 coefficient is finite
     float x_inv_scale;    // int8 + x_nchw_f32 explicit path: quantise while packing
     int y_nchw;           // y is fp32 in the reference layout
     int w_const;          // w holds weights prepared before this call
@@ -516,6 +519,7 @@ int run_conv(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &
     p.residual = io.residual; p.res_relu = io.res_relu; p.round_tf32 = io.round_tf32;
     p.lut_smem = p.act == SILU && p.lut && !p.residual && (reinterpret_cast<uintptr_t>(p.lut) & 15) == 0;
     p.out_q = io.out_q; p.q_inv_scale = io.q_inv_scale;
+    p.q_table = pl.kind == KIND_I8 && io.coeff_finite && fabsf(e.in_scale) < 0x1p90f;
     p.status = ctx->status_dev;
     UnitParams u;
     memset(&u, 0, sizeof(u));
@@ -994,6 +998,7 @@ struct one_packed {
     ConvPlan pl;
     // Gemm / MatMul
     int M, K, N, Kp, b_shared, bn, auto_tile;
+    int coeff_finite = 0;
     // device-resident constants
     void *w = nullptr;
     void *bias = nullptr;
@@ -1111,6 +1116,7 @@ static int prepare_conv(one_packed *op, BUFFER_INFO_S *params, BUFFER_INFO_S *in
     if (op->e.int8) {
         std::vector<float> coeff;
         dequant_coeffs(cfg, g.OC, &coeff);
+        op->coeff_finite = std::all_of(coeff.begin(), coeff.end(), [](float c) { return std::isfinite(c); });
         if ((rc = upload(reinterpret_cast<void **>(&op->coeff), coeff.data(), (size_t)g.OC * 4)) != ONE_OK) return rc;
     }
     if (op->e.act == SILU) {
@@ -1239,7 +1245,7 @@ extern "C" int one_cuda_eval_async(one_ctx *ctx, one_packed *op, BUFFER_INFO_S *
         ConvIO io;
         memset(&io, 0, sizeof(io));
         io.w = op->w; io.bias = op->bias; io.coeff = op->coeff; io.lut = op->lut;
-        io.w_const = 1;
+        io.w_const = 1; io.coeff_finite = op->coeff_finite;
         const float inv_scale = op->e.int8 ? 1.0f / op->e.in_scale : 1.f;
         cudaError_t ce;
         int rc;

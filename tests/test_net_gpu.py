@@ -649,3 +649,43 @@ def n_trace_details(n):
         n.trace(p, runs=1)
         rows = [ln.split(",") for ln in open(p).read().strip().split("\n")[1:]]
     return {r[0]: r[13] for r in rows}
+
+
+@pytest.mark.parametrize("scale", [0.002, 0.03, 0.2, 20.0])
+def test_int8_output_of_a_table_activation_bit_exact_at_every_scale_range(oracle_mod, scale):
+    """The epilogue that looks quantised bytes up has one form per range of the reader's scale (values of 8 and more all
+    saturate, or do not, or 8 rounds to nothing; the first entry rounds to 0 or not); sums of at most 256 products (the
+    stem, the 1 x 1) and longer ones; pre-activations on both sides of the table.  Integers: bit exact."""
+    from onenew_b200 import abi, quant
+    from onenew_b200.one_file import OneBuilder
+    rng = np.random.default_rng(77)
+    IM = 402                                          # 201 x 201 pixels per layer: 316 row tiles, the last one ragged
+    stack = [(3, 64, 3, 2, 1), (64, 64, 1, 1, 0), (64, 96, 3, 1, 1), (96, 32, 1, 1, 0)]
+    b = OneBuilder()
+    b.add_io("input", "input", (1, 3, IM, IM))
+    x, hw, ws = "input", IM, []
+    for i, (ci, co, k, s, p) in enumerate(stack):
+        w = (rng.standard_normal((co, ci, k, k)) * 6.0 / np.sqrt(ci * k * k)).astype(np.float32)
+        bias = (rng.standard_normal(co) * 4.0).astype(np.float32)
+        ws.append((w, bias))
+        out = "output" if i == len(stack) - 1 else f"Conv_{i}_out"
+        b.conv(f"Conv_{i}", x, b.add_init(f"Conv_{i}.weight", w), b.add_init(f"Conv_{i}.bias", bias), out, (k, k), (s, s), (p,) * 4,
+               act=abi.SILU if i < len(stack) - 1 else abi.NOT_ACT)
+        hw = (hw + 2 * p - k) // s + 1
+        x = out
+    b.add_io("output", "output", (1, stack[-1][1], hw, hw))
+    scales = {f"Conv_{i}": np.float32(1 / 127 if i == 0 else scale) for i in range(len(stack))}
+    n = onet.Net(quant.quantize_model(b.tobytes(), scales), batch=1)
+    try:
+        cur = rng.uniform(0, 1, (1, 3, IM, IM)).astype(np.float32)
+        y = n(cur)
+        for i, ((ci, co, k, s, p), (w, bias)) in enumerate(zip(stack, ws)):
+            w8, b32, aux = oracle_mod.quant_weight_bias(w, bias)
+            last = i == len(stack) - 1
+            cur = oracle_mod.conv_s8(cur, w8, b32, aux, float(scales[f"Conv_{i}"]), (s, s), p, abi.NOT_ACT if last else abi.SILU)[0]
+            if not last:
+                q = n.fetch(f"Conv_{i}_out", cur.shape)
+                assert np.array_equal(q, oracle_mod.quantize_s8(cur, scale).astype(np.float32)), f"Conv_{i}_out"
+        assert np.array_equal(y, cur)
+    finally:
+        n.close()
