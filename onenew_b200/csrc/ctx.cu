@@ -7,6 +7,7 @@
 #include <atomic>
 #include <map>
 #include <mutex>
+#include <vector>
 
 #include "../../include/one_cuda.h"
 
@@ -51,40 +52,48 @@ void *ws_alloc(one_ctx *c, size_t bytes)
     return c->ws + off;
 }
 
-// Status words are slots of one mapped page that lives as long as the process (pinning a page takes ~10 ms, too long
-// for every context); a context gives its slot back when it is released.  More contexts than slots: an error.
+// Status words are slots of mapped pages that live as long as the process (pinning a page takes ~10 ms, too long for
+// every context); a context gives its slot back when it is released, and another page is pinned only when all are taken.
+struct StatusPage {
+    static constexpr size_t SLOTS = 1024;
+    unsigned int *words = nullptr;
+    bool used[SLOTS] = {};
+};
 static std::mutex g_slot_mu;
-static unsigned int *g_slots = nullptr;
-static bool g_slot_used[1024];
+static std::vector<StatusPage *> g_status_pages;
 
 static cudaError_t status_slot_take(unsigned int **host, unsigned int **dev)
 {
     std::lock_guard<std::mutex> lk(g_slot_mu);
-    if (!g_slots) {
-        void *p = nullptr;
-        cudaError_t e = cudaHostAlloc(&p, sizeof(g_slot_used) * sizeof(unsigned int), cudaHostAllocMapped | cudaHostAllocPortable);
-        if (e != cudaSuccess) return e;
-        g_slots = static_cast<unsigned int *>(p);
+    for (size_t page = 0;; ++page) {
+        if (page == g_status_pages.size()) {
+            void *p = nullptr;
+            cudaError_t e = cudaHostAlloc(&p, StatusPage::SLOTS * sizeof(unsigned int), cudaHostAllocMapped | cudaHostAllocPortable);
+            if (e != cudaSuccess) return e;
+            g_status_pages.push_back(new StatusPage);
+            g_status_pages.back()->words = static_cast<unsigned int *>(p);
+        }
+        StatusPage *pg = g_status_pages[page];
+        for (size_t i = 0; i < StatusPage::SLOTS; ++i) {
+            if (pg->used[i]) continue;
+            void *d = nullptr;
+            cudaError_t e = cudaHostGetDevicePointer(&d, pg->words + i, 0);
+            if (e != cudaSuccess) return e;
+            pg->used[i] = true;
+            pg->words[i] = 0;
+            *host = pg->words + i;
+            *dev = static_cast<unsigned int *>(d);
+            return cudaSuccess;
+        }
     }
-    for (size_t i = 0; i < sizeof(g_slot_used); ++i) {
-        if (g_slot_used[i]) continue;
-        void *d = nullptr;
-        cudaError_t e = cudaHostGetDevicePointer(&d, g_slots + i, 0);
-        if (e != cudaSuccess) return e;
-        g_slot_used[i] = true;
-        g_slots[i] = 0;
-        *host = g_slots + i;
-        *dev = static_cast<unsigned int *>(d);
-        return cudaSuccess;
-    }
-    return cudaErrorMemoryAllocation;
 }
 
 static void status_slot_give(const volatile unsigned int *host)
 {
     if (!host) return;
     std::lock_guard<std::mutex> lk(g_slot_mu);
-    g_slot_used[host - g_slots] = false;
+    for (StatusPage *pg : g_status_pages)
+        if (host >= pg->words && host < pg->words + StatusPage::SLOTS) pg->used[host - pg->words] = false;
 }
 
 int take_status(one_ctx *c)
