@@ -311,35 +311,61 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     const bool in = row < rows && k + e < u.K;
                     v[e] = in ? __ldg(mode == 2 ? base + (long long)(k + e) * pitch + row : base + (long long)row * pitch + k + e) : 0.f;
                 }
-                return rnd4(make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3])));
+                return make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
             };
+            // A plainly loaded B tile is fetched into registers one K block ahead: its latency runs under the current block.
+            // Lanes run along the rows for a [K][rows] operand and along K for K-major rows: coalesced either way.
+            constexpr int BPIECES = (BN * 8 + 191) / 192;
+            uint4 bnext[BPIECES];
+            const int cshift = 31 - __clz(cpr);
+            auto piece_b = [&](int j, int &r, int &c) {
+                r = u.b_ld == 2 ? j % BN : j >> cshift;
+                c = u.b_ld == 2 ? j / BN : j & (cpr - 1);
+            };
+            auto fetch_b = [&](int i) {
+                const float *base = u.b + (long long)bz * u.b_bstride;
+#pragma unroll
+                for (int q = 0; q < BPIECES; ++q) {
+                    int r, c;
+                    piece_b(t + 192 * q, r, c);
+                    if (t + 192 * q < BN * cpr) bnext[q] = fetch(base, u.b_ld, u.b_pitch, n0 + r, p.N, (kb0 + i) * p.slab_elems + 4 * c);
+                }
+            };
+            if (u.b_ld) fetch_b(0);
             uint32_t s = 0, phase = 0;   // ring slot, and the phase of its `full`
             for (int i = 0; i < nkb && ok; ++i) {
                 uint8_t *st = smem + s * stage_bytes;
                 const int k0 = (kb0 + i) * p.slab_elems;
                 if ((u.a_ld || u.b_ld) && i >= stages && !mbar_wait(empty0 + 8 * s, phase ^ 1, abort_flag)) ok = false;
-                // lanes run along the rows for a [K][rows] operand and along K for K-major rows: coalesced either way
                 if (ok && u.a_ld) {
                     const float *base = u.a + (long long)bz * u.a_bstride;
+#pragma unroll 3
                     for (int j = t; j < A_ROWS * cpr; j += 192) {
-                        const int r = j / cpr, c = j - r * cpr;
-                        *reinterpret_cast<uint4 *>(st + r * p.slab_bytes + (slot_of(r, c) << 4)) = fetch(base, 1, u.a_pitch, m0 + r, p.M, k0 + 4 * c);
+                        const int r = j >> cshift, c = j & (cpr - 1);
+                        *reinterpret_cast<uint4 *>(st + r * p.slab_bytes + (slot_of(r, c) << 4)) = rnd4(fetch(base, 1, u.a_pitch, m0 + r, p.M, k0 + 4 * c));
                     }
                 }
                 if (ok && u.b_ld) {
-                    const float *base = u.b + (long long)bz * u.b_bstride;
-                    for (int j = t; j < BN * cpr; j += 192) {
-                        const int r = u.b_ld == 2 ? j % BN : j / cpr, c = u.b_ld == 2 ? j / BN : j - r * cpr;
-                        *reinterpret_cast<uint4 *>(st + a_slab + r * p.slab_bytes + (slot_of(r, c) << 4)) = fetch(base, u.b_ld, u.b_pitch, n0 + r, p.N, k0 + 4 * c);
+#pragma unroll
+                    for (int q = 0; q < BPIECES; ++q) {
+                        int r, c;
+                        piece_b(t + 192 * q, r, c);
+                        if (t + 192 * q < BN * cpr) *reinterpret_cast<uint4 *>(st + a_slab + r * p.slab_bytes + (slot_of(r, c) << 4)) = rnd4(bnext[q]);
                     }
+                    if (i + 1 < nkb) fetch_b(i + 1);
                 }
                 if (ok && tx) {
                     if (!mbar_wait(full0 + 8 * s, phase, abort_flag)) ok = false;
                     else {
                         const uint32_t lo = tma_a ? 0u : a_slab, hi = tma_b ? stage_bytes : a_slab;
-                        for (uint32_t o = lo + 16u * t; o < hi; o += 16u * 192u) {
-                            uint4 *q = reinterpret_cast<uint4 *>(st + o);
-                            *q = rnd4(*q);
+                        for (uint32_t o = lo + 16u * t; o < hi; o += 4u * 16u * 192u) {   // four pieces in flight
+                            uint4 v[4];
+#pragma unroll
+                            for (uint32_t e = 0; e < 4; ++e)
+                                if (o + e * 3072u < hi) v[e] = *reinterpret_cast<uint4 *>(st + o + e * 3072u);
+#pragma unroll
+                            for (uint32_t e = 0; e < 4; ++e)
+                                if (o + e * 3072u < hi) *reinterpret_cast<uint4 *>(st + o + e * 3072u) = rnd4(v[e]);
                         }
                     }
                 }
