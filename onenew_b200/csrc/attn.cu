@@ -11,8 +11,12 @@
 // touches HBM: the kernel reads the fused qkv tensor [B][T][3*D] once and writes ctx [B][T][D].
 //
 // One CTA per (image, head, 128-query-row tile), two CTAs resident per SM so that one CTA's loads
-// and MMAs overlap the other's softmax.  Warp 4 issues TMA and tcgen05.mma; warps 0-3 own one TMEM
-// lane quarter each (32 query rows) and do the softmax and the epilogue.
+// and MMAs overlap the other's softmax.  Warp 8 issues TMA and tcgen05.mma; warps 0-7 do the softmax and
+// the epilogue: warps q and q + 4 share TMEM lane quarter q (32 query rows) and take alternate 32-column
+// blocks, exchanging row maxima and sums through shared memory.  What bounds the kernel is the dependency
+// chain of a tile, and about half of that is the softmax: one warp per quarter walked 7 blocks of a
+// 197-token row twice with nothing to hide its latencies (10 warps on an SM, no pipe above 21 %).  Two halve
+// the walk.  A quarter that lies past the last token hands its blocks over unwritten: nothing reads those rows.
 //   1. TMA: Q tile [128][hd] and K [T16][hd] straight out of the qkv tensor (the head split is the
 //      tensor map's column coordinate; rows past T are zero-filled), 128-byte swizzle.
 //   2. S = Q K^T: M = 128, N = T16, K = hd; both operands K-major; accumulator in TMEM columns [0, T16).
@@ -49,7 +53,9 @@ struct AttnParams {
 
 namespace {
 
-constexpr int ATTN_THREADS = 160;
+constexpr int ATTN_THREADS = 288;
+constexpr int MMA_WARP = 8;
+constexpr uint32_t XCHG_BYTES = 2 * 2 * 128 * 4;   // row maxima and row sums of both column halves
 constexpr uint32_t TMEM_COLS = 256;
 constexpr int MAX_RING = 3;
 
@@ -86,7 +92,8 @@ attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     // region shared in time: first Q | K, then V | ring of P blocks, then the output patches
     uint8_t *sQ = smem, *sK = smem + q_bytes, *sV = smem, *sRing = smem + v_bytes;
     const uint32_t qk = q_bytes + k_bytes, vr = v_bytes + (uint32_t)p.ring * 16384u;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (qk > vr ? qk : vr));
+    float *xmax = reinterpret_cast<float *>(smem + (qk > vr ? qk : vr)), *xsum = xmax + 256;   // [half][row]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (qk > vr ? qk : vr) + XCHG_BYTES);
     // barriers: qk, v, s, o, full[MAX_RING], empty[MAX_RING]
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 4 + 2 * MAX_RING);
     int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
@@ -109,12 +116,12 @@ attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
         mbar_init(bar_s, 1);
         mbar_init(bar_o, 1);
         for (int s = 0; s < MAX_RING; ++s) {
-            mbar_init(full0 + 8 * s, 4);    // one arrival per softmax warp
+            mbar_init(full0 + 8 * s, 4);    // one arrival per warp of the half that writes the block
             mbar_init(empty0 + 8 * s, 1);   // tcgen05.commit
         }
         fence_mbar_init();
     }
-    if (warp == 4) {
+    if (warp == MMA_WARP) {
         tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
         tmem_relinquish();
     }
@@ -126,7 +133,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     pdl_wait();
 
     bool v_issued = false;
-    if (warp == 4) {
+    if (warp == MMA_WARP) {
         // ------------------------------------------------------------ TMA + MMA issue
         if (lane == 0) {
             mbar_arrive_expect_tx(bar_qk, q_bytes + k_bytes);
@@ -193,98 +200,98 @@ attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
         }
         if (!ok && lane == 0) atomicOr(p.status, ST_TIMEOUT_MMA);
     } else {
-        // ------------------------------------------------------------ softmax + epilogue (warps 0-3)
-        const int row = 32 * warp + lane;              // accumulator row (TMEM lane) of this thread
-        const uint32_t t_row = tmem_base + ((uint32_t)(32 * warp) << 16);
+        // ------------------------------------------------------------ softmax + epilogue (warps 0-7)
+        const int quarter = warp & 3, half = warp >> 2;
+        const int row = 32 * quarter + lane;           // accumulator row (TMEM lane) of this thread
+        const uint32_t t_row = tmem_base + ((uint32_t)(32 * quarter) << 16);
+        const bool live = m0 + 32 * quarter < p.T;     // (the same for both warps of the quarter)
+        auto pair_sync = [&]() {
+            __syncwarp();
+            asm volatile("barrier.sync %0, 64;" ::"r"(1 + quarter) : "memory");
+        };
         bool ok = mbar_wait(bar_s, 0, abort_flag);
-        float sum = 0.f;
-        if (ok) {
+        // Two passes over this half's blocks of the accumulator row in TMEM, 32 columns at a time; the running
+        // maximum / sum are kept in four independent chains.
+        uint32_t v[32];
+        float mx4[4] = {-32768.0f, -32768.0f, -32768.0f, -32768.0f};   // softmax.c:53
+        if (ok && live) {
             tc_fence_after_sync();
-            // Two passes over the accumulator row in TMEM, 32 columns at a time.  The load of the next
-            // block is in flight while the current one is processed (two register buffers), and the
-            // running maximum / sum are kept in four independent chains.
-            uint32_t va[32], vb[32];
-            float mx4[4] = {-32768.0f, -32768.0f, -32768.0f, -32768.0f};   // softmax.c:53
-            auto pass1 = [&](const uint32_t (&v)[32], int c) {
-                const int lim = p.T - 32 * c;
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (j < lim) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(v[j]));
-            };
-            tmem_ld_32x32(t_row, va);
-            for (int c = 0; c < chunks; c += 2) {
+            for (int c = half; c < chunks; c += 2) {
+                tmem_ld_32x32(t_row + 32 * c, v);
                 tmem_ld_wait();
-                if (c + 1 < chunks) tmem_ld_32x32(t_row + 32 * (c + 1), vb);
-                pass1(va, c);
-                if (c + 1 < chunks) {
-                    tmem_ld_wait();
-                    if (c + 2 < chunks) tmem_ld_32x32(t_row + 32 * (c + 2), va);
-                    pass1(vb, c + 1);
+                const int lim = p.T - 32 * c;
+                if (lim >= 32) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(v[j]));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if (j < lim) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(v[j]));
                 }
             }
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            // exp(scale * (s - max)) as 2^(s * a - b)
-            const float a2 = p.scale * 1.4426950408889634f, b2 = mx * a2;
-            float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-            auto pass2 = [&](const uint32_t (&v)[32], int c) -> bool {
-                const int lim = p.T - 32 * c;
-                float e[32];
+            tc_fence_before_sync();
+        }
+        xmax[half * 128 + row] = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+        pair_sync();
+        const float mx = fmaxf(xmax[row], xmax[128 + row]);
+        // exp(scale * (s - max)) as 2^(s * a - b)
+        const float a2 = p.scale * 1.4426950408889634f, b2 = mx * a2;
+        float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int c = half; c < chunks && ok; c += 2) {
+            const int s = c % NR, lim = p.T - 32 * c;
+            float e[32];
+            if (live) {
+                tmem_ld_32x32(t_row + 32 * c, v);
+                tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const float t = ex2_approx(fmaf(__uint_as_float(v[j]), a2, -b2));
-                    e[j] = (j < lim) ? t : 0.f;
-                    sum4[j & 3] += e[j];
+                for (int j = 0; j < 32; ++j) e[j] = ex2_approx(fmaf(__uint_as_float(v[j]), a2, -b2));
+                if (lim < 32) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) e[j] = j < lim ? e[j] : 0.f;
                 }
-                const int s = c % NR;
-                // the ring slot is free once the MMAs that read its previous block have completed
-                if (c >= NR && !mbar_wait(empty0 + 8 * s, (uint32_t)((c / NR - 1) & 1), abort_flag)) return false;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) sum4[j & 3] += e[j];
+            }
+            // the ring slot is free once the MMAs that read its previous block have completed
+            if (c >= NR && !mbar_wait(empty0 + 8 * s, (uint32_t)((c / NR - 1) & 1), abort_flag)) {
+                ok = false;
+                break;
+            }
+            if (live) {
                 uint8_t *prow = sRing + s * 16384 + row * 128;
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     *reinterpret_cast<float4 *>(prow + ((j ^ (row & 7)) << 4)) = make_float4(e[4 * j], e[4 * j + 1], e[4 * j + 2], e[4 * j + 3]);
-                tc_fence_before_sync();     // this block of S has been read (the first blocks are overwritten by O)
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full0 + 8 * s);
-                return true;
-            };
-            tmem_ld_32x32(t_row, va);
-            for (int c = 0; c < chunks && ok; c += 2) {
-                tmem_ld_wait();
-                if (c + 1 < chunks) tmem_ld_32x32(t_row + 32 * (c + 1), vb);
-                ok = pass2(va, c);
-                if (ok && c + 1 < chunks) {
-                    tmem_ld_wait();
-                    if (c + 2 < chunks) tmem_ld_32x32(t_row + 32 * (c + 2), va);
-                    ok = pass2(vb, c + 1);
-                }
             }
-            tmem_ld_wait();
-            sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-            if (ok) ok = mbar_wait(bar_o, 0, abort_flag);
+            tc_fence_before_sync();     // this block of S has been read (the first blocks are overwritten by O)
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full0 + 8 * s);
         }
+        xsum[half * 128 + row] = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+        if (ok) ok = mbar_wait(bar_o, 0, abort_flag);
+        pair_sync();
         if (ok) {
-            tc_fence_after_sync();
-            const float inv = 1.0f / sum;
-            uint8_t *patch = smem + warp * (hdb * 4096);   // V and the ring are dead once O is complete
-            uint32_t v[32];
-            for (int cb = 0; cb < hdb; ++cb) {
-                tmem_ld_32x32(t_row + 32 * cb, v);
+            // each half finishes one 32-column block of O (the only one of a 32-wide head: the first half)
+            if (live && half < hdb) {
+                tc_fence_after_sync();
+                const float inv = 1.0f / (xsum[row] + xsum[128 + row]);
+                uint8_t *patch = smem + (quarter * hdb + half) * 4096;   // V and the ring are dead once O is complete
+                tmem_ld_32x32(t_row + 32 * half, v);
                 tmem_ld_wait();
-                uint8_t *prow = patch + cb * 4096 + lane * 128;
+                uint8_t *prow = patch + lane * 128;
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     *reinterpret_cast<float4 *>(prow + ((j ^ (lane & 7)) << 4)) =
                         make_float4(__uint_as_float(v[4 * j]) * inv, __uint_as_float(v[4 * j + 1]) * inv,
                                     __uint_as_float(v[4 * j + 2]) * inv, __uint_as_float(v[4 * j + 3]) * inv);
-            }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0 && m0 + 32 * warp < p.T) {
-                for (int cb = 0; cb < hdb; ++cb)
-                    tma_store_3d(&tmO, smem_u32(patch + cb * 4096), h * p.hd + cb * 32, m0 + 32 * warp, img);
-                bulk_commit();
-                bulk_wait_read0();
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_3d(&tmO, smem_u32(patch), h * p.hd + half * 32, m0 + 32 * quarter, img);
+                    bulk_commit();
+                    bulk_wait_read0();
+                }
             }
         } else if (lane == 0) {
             atomicOr(p.status, ST_TIMEOUT_EPILOGUE);
@@ -294,7 +301,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     // ------------------------------------------------------------ teardown
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 4) {
+    if (warp == MMA_WARP) {
         if (*abort_flag) {   // let a load in flight land before the shared memory is given back
             int dummy = 0;
             if (!(mbar_wait(bar_qk, 0, &dummy) && (!v_issued || mbar_wait(bar_v, 0, &dummy))) && lane == 0)
@@ -332,10 +339,10 @@ extern "C" int one_cuda_attention(one_ctx *ctx, const float *qkv, float *out, in
     p.status = ctx->status_dev;
     const int hdb = hd / 32;
     const size_t qk = (size_t)hdb * (128 + p.tp16) * 128, vb = (size_t)hdb * p.tp8 * 128;
-    // three ring slots when two CTAs still fit an SM with them, else two
-    p.ring = (1024 + (vb + 3 * 16384 > qk ? vb + 3 * 16384 : qk) + 128) * 2 <= 227 * 1024 ? 3 : 2;
+    // three ring slots when two CTAs still fit an SM with them (228 KB, of which a CTA costs 1 KB by itself), else two
+    p.ring = (1024 + (vb + 3 * 16384 > qk ? vb + 3 * 16384 : qk) + XCHG_BYTES + 128 + 1024) * 2 <= 228 * 1024 ? 3 : 2;
     const size_t vr = vb + (size_t)p.ring * 16384;
-    const size_t smem = 1024 + (qk > vr ? qk : vr) + 128;
+    const size_t smem = 1024 + (qk > vr ? qk : vr) + XCHG_BYTES + 128;
     if (smem > 227 * 1024) return fail(ONE_ERR_UNSUPPORTED, "attention: %zu bytes of shared memory needed", smem);
     CUtensorMap tmQ, tmK, tmV, tmO;
     const uint64_t pitch = (uint64_t)row_floats * 4, bpitch = pitch * T;
