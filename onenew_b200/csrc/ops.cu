@@ -105,6 +105,27 @@ inline int kind_tm(int kind) { return kind == KIND_TF32 ? TM_F32 : (kind == KIND
 inline int kind_of_prec(int prec) { return prec == ONE_PREC_BF16 ? KIND_BF16 : (prec == ONE_PREC_F16 ? KIND_F16 : KIND_TF32); }
 inline bool valid_prec(int prec) { return prec == ONE_PREC_TF32 || prec == ONE_PREC_BF16 || prec == ONE_PREC_F16; }
 inline int kind_out16(int kind) { return kind == KIND_F16 ? OUT_F16 : OUT_BF16; }   // the kind's own 16-bit output mode
+// How the tiles of width `bn` are walked when the library chooses (`taps`: a filter of several positions; 0 a plain product;
+// c_slabs: K blocks per filter position).  Every form gives the same sums; they differ in what bounds a launch of many tiles.
+// Until now only a tile search chose them.  Whole networks, us, single CTAs -> this rule: int8 backbone of 64 images
+// 1955 -> 1625, ResNet-50 fp16 256 images 4837 -> 4535, ViT-Tiny 256 images 3555 -> 3485, ResNet-50 TF32 61 images equal.
+//  * 64 wide: operand traffic and barrier hand-overs -- two 128-row halves against one tile of B.  TF32 products of few K
+//    blocks are bound by HBM instead and stay plain.
+//  * 128 wide, 3x3 filters of enough channels: the same; from about a wave on, since halves also shorten a ragged last wave.
+//  * 256 / 128 wide with 8 K blocks or more: the operand stream -- pairs of CTAs, which load half of B each.
+//  * int8 with at most 4 K blocks: the epilogue -- twelve warps of it behind a shallower ring.
+inline int refine_tile(int code, int kind, long long M, int N, int num_kb, bool taps, int c_slabs)
+{
+    if (code >= 1000 || valid_tile(t_tile_n)) return code;
+    const bool half = g_half_tiles.load(std::memory_order_relaxed), pair = g_cta_pairs.load(std::memory_order_relaxed), wide = g_wide_epi.load(std::memory_order_relaxed);
+    const long long m_tiles = (M + 127) / 128, tiles = m_tiles * ((N + code - 1) / code), SMS = 148;
+    if (code == 64) return half && tiles >= 4 * SMS && (kind != KIND_TF32 || taps) ? 2064 : code;
+    if (kind == KIND_I8) return wide && !taps && num_kb <= 4 && m_tiles * ((N + 127) / 128) >= 2 * SMS ? 4128 : code;
+    if (code == 128 && taps) return half && tiles >= SMS && c_slabs >= (kind == KIND_TF32 ? 4 : 2) ? 2128 : code;
+    if (code == 128) return pair && num_kb >= 8 && tiles >= 8 * SMS ? 1128 : code;
+    if (code == 256) return pair && num_kb >= 8 && tiles >= 2 * SMS ? 1256 : code;
+    return code;
+}
 inline const char *kind_name(int kind) { return kind == KIND_I8 ? "s8" : (kind == KIND_BF16 ? "bf16" : (kind == KIND_F16 ? "f16" : "tf32")); }
 inline int slab_for_bytes(long long row_bytes) { return row_bytes >= 128 ? 128 : (row_bytes >= 64 ? 64 : 32); }
 
@@ -330,7 +351,8 @@ void plan_conv(const ConvGeom &g, int kind, ConvPlan *p, bool x_nchw_f32)
         p->c_slabs = p->num_kb;
     }
     p->slab_elems = p->slab_bytes / p->es;
-    const int code = pick_bn(g.OC, (long long)g.N * g.OH * g.OW);
+    const int code = refine_tile(pick_bn(g.OC, (long long)g.N * g.OH * g.OW), kind, (long long)g.N * g.OH * g.OW, g.OC, p->num_kb,
+                                 p->path == PATH_IM2COL || p->path == PATH_S2D, p->c_slabs);
     p->bn = tile_bn(code);
     p->cta2 = tile_cta2(code) ? 1 : 0;
     p->mh = tile_mh(code);
@@ -1206,7 +1228,11 @@ static int prepare_gemm(one_packed *op, bool is_gemm, BUFFER_INFO_S *params, BUF
         const OPERAND_S *a0 = reinterpret_cast<const OPERAND_S *>(params[1].addr);
         long long rows = 1;
         for (int i = 0; i < a0->dim_num_of_shapes - 1 && i < SHAPE_LEN; ++i) rows *= a0->shapes[i];
-        op->bn = pick_bn(op->N, rows);
+        op->bn = refine_tile(pick_bn(op->N, rows), op->kind, rows, op->N, (int)(((long long)op->K * es + 127) / 128), false, 1);
+        // ViT-Tiny's widths: pairs when the rows are many (qkv, fc2)
+        if (op->bn == 192 && !valid_tile(t_tile_n) && g_cta_pairs.load(std::memory_order_relaxed) && op->kind == KIND_TF32 && (long long)op->K * es >= 6 * 128 &&
+            (rows + 127) / 128 * ((op->N + 191) / 192) >= 2 * 148)
+            op->bn = 1192;
         op->auto_tile = !valid_tile(t_tile_n);
     }
     if ((rc = upload(tmp, reinterpret_cast<const void *>(inputs[1].addr), (size_t)op->K * op->N * 4)) != ONE_OK) return rc;

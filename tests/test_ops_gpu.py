@@ -548,3 +548,39 @@ def test_one_wave_conv_vs_oracle_and_persistent(ops, oracle_mod, case):
     assert_close(z, ref, "persistent")
     ref8 = oracle_mod.conv_s8(x, w8, b32, aux, 0.01, (s, s), p, act)[0]
     assert np.array_equal(y8, ref8) and np.array_equal(z8, ref8)
+
+
+# precision, N, C, H, W, OC, k, stride, the plain tile: one launch of each form that the library chooses by itself, just
+# above the size from which it does
+CHOSEN_FORMS = [
+    ("int8", 1, 3, 560, 560, 32, 3, 2, 64), ("int8", 1, 128, 200, 200, 128, 1, 1, 128), ("f16", 1, 128, 150, 151, 128, 3, 1, 128),
+    ("f16", 1, 512, 390, 390, 128, 1, 1, 128), ("f16", 1, 512, 195, 195, 256, 1, 1, 256), ("tf32", 1, 3, 560, 562, 48, 7, 2, 64),
+]
+
+
+@pytest.mark.parametrize("case", CHOSEN_FORMS, ids=[f"{c[0]}_{c[2]}to{c[5]}k{c[6]}@{c[3]}x{c[4]}" for c in CHOSEN_FORMS])
+def test_chosen_tile_form_equals_plain_tiles(ops, oracle_mod, case):
+    """Halves, pairs and twelve epilogue warps add the same products in the same order as single CTAs: the same bits."""
+    import torch
+    prec, N, C, H, W, OC, k, s, tile = case
+    gen = torch.Generator(device="cuda").manual_seed(C + OC + H)
+    x = torch.rand((N, C, H, W), generator=gen, device="cuda") * 2 - 1
+    w = (torch.randn((OC, C, k, k), generator=gen, device="cuda") * 0.05).cpu().numpy()
+    b = (torch.randn((OC,), generator=gen, device="cuda") * 0.1).cpu().numpy()
+    L = capi.lib()
+
+    def run():
+        if prec == "int8":
+            w8, b32, aux = oracle_mod.quant_weight_bias(w, b)
+            return ops.conv(x, w8, b32, (s, s), (k // 2,) * 4, abi.RELU, int8=(0.01, aux))
+        return ops.conv(x, w, b, (s, s), (k // 2,) * 4, abi.RELU)
+
+    capi.check(L.one_cuda_set_eval_precision(capi.PRECISIONS["tf32" if prec == "int8" else prec]))
+    try:
+        y = run()
+        capi.check(L.one_cuda_set_tile_n(tile))
+        z = run()
+    finally:
+        L.one_cuda_set_tile_n(0)
+        L.one_cuda_set_eval_precision(capi.PREC_TF32)
+    assert torch.equal(y, z) and bool(y.any())
