@@ -170,11 +170,13 @@ ONE_API int one_cuda_set_tile_n(int bn);
  * tiles would occupy at most half the SMs cuts its K range into several pieces, each piece accumulated
  * by its own CTA into a scratch plane, the planes added in a fixed order by a second short kernel that
  * also applies bias / activation / residual), 1 = never split, 2..64 = that many pieces when the shape
- * allows it.  Only the float paths split; results do not depend on scheduling. */
+ * allows it.  Only the float paths split that way; results do not depend on scheduling.  With 0, and no tile
+ * override, a launch whose 128 x 64 tiles are all resident at once runs one tile per CTA instead, its K range
+ * shared by a cluster of up to eight CTAs; 1 therefore also gives sums that do not depend on the batch. */
 ONE_API int one_cuda_set_split_k(int splits);
 /* The same choice for one prepared operator (0: follow the calling thread's setting); used by the tile search. */
 ONE_API int one_cuda_packed_set_split(one_packed *op, int splits);
-/* Process-wide switch (default on) for launching the contraction kernels with programmatic stream
+/* Process-wide switch (default on) for launching the library's kernels with programmatic stream
  * serialisation: a kernel may be scheduled while the previous kernel on its stream drains, runs its
  * set-up (barriers, tensor memory, descriptor prefetch) and then waits on the device until that
  * previous kernel has completed before it touches any tensor. */
