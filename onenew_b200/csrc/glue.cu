@@ -92,6 +92,47 @@ __global__ void k_nhwc_to_nchw(const T *__restrict__ x, float *__restrict__ y, i
     }
 }
 
+// The same for whole groups of four channels: a block moves 32 pixels x 128 channels with 4 channels a load and four loads
+// in flight per thread (the form above has one value a load: 42 us for the 105 MB of a detector's last layer, whose floor
+// is 16).  In shared memory 4-channel piece j of pixel p lies at j ^ (p & 7): a lane writes and reads 16 bytes without
+// conflicts, and a warp's store covers 32 consecutive pixels of one channel.  int8 backbone of 64 images 1625 -> 1603 us,
+// of one image 119 -> 117.
+template <typename T> struct alignas(4 * sizeof(T)) Four { T v[4]; };
+template <typename T>
+__global__ void __launch_bounds__(256) k_nhwc_to_nchw4(const T *__restrict__ x, float *__restrict__ y, int C, int HW)
+{
+    pdl_entry(x);
+    __shared__ float4 tile[32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = blockIdx.z, c0 = blockIdx.y * 128, p0 = blockIdx.x * 32;
+    const T *xi = x + (size_t)n * C * HW;
+    float *yo = y + (size_t)n * C * HW;
+    Four<T> q[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int p = p0 + warp + 8 * k, c = c0 + 4 * lane;
+        if (p < HW && c < C) q[k] = *reinterpret_cast<const Four<T> *>(xi + (size_t)p * C + c);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int r = warp + 8 * k, c = c0 + 4 * lane;
+        if (p0 + r < HW && c < C) tile[r][lane ^ (r & 7)] = make_float4(Cvt<T>::to(q[k].v[0]), Cvt<T>::to(q[k].v[1]), Cvt<T>::to(q[k].v[2]), Cvt<T>::to(q[k].v[3]));
+    }
+    __syncthreads();
+    if (p0 + lane >= HW) return;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int j = warp + 8 * k, c = c0 + 4 * j;
+        if (c >= C) break;
+        const float4 f = tile[lane][j ^ (lane & 7)];
+        float *o = yo + (size_t)c * HW + p0 + lane;
+        o[0] = f.x;
+        o[HW] = f.y;
+        o[2 * (size_t)HW] = f.z;
+        o[3 * (size_t)HW] = f.w;
+    }
+}
+
 cudaError_t nchw_to_nhwc(const float *x, void *y, int N, int C, int HW, int dt, int round_tf32, float inv_scale,
                          cudaStream_t s)
 {
@@ -109,6 +150,15 @@ cudaError_t nhwc_to_nchw(const void *x, float *y, int N, int C, int HW, int dt, 
 {
     if (N <= 0 || C <= 0 || HW <= 0) return cudaSuccess;
     dim3 grid((HW + 31) / 32, (C + 31) / 32, N), block(32, 8);
+    // Whole, aligned groups of four channels, and enough of them to fill half of a block's lanes: the wide form.
+    if (C >= 64 && (C & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (dt == DT_F32 || dt == DT_BF16 || dt == DT_F16)) {
+        const dim3 g4((HW + 31) / 32, (C + 127) / 128, N);
+        if (dt == DT_F32) launch_k(k_nhwc_to_nchw4<float>, g4, 256, 0, s, (const float *)x, y, C, HW);
+        else if (dt == DT_BF16) launch_k(k_nhwc_to_nchw4<__nv_bfloat16>, g4, 256, 0, s, (const __nv_bfloat16 *)x, y, C, HW);
+        else launch_k(k_nhwc_to_nchw4<__half>, g4, 256, 0, s, (const __half *)x, y, C, HW);
+        count_launch();
+        return cudaGetLastError();
+    }
     if (dt == DT_F32) launch_k(k_nhwc_to_nchw<float>, grid, block, 0, s, (const float *)x, y, C, HW);
     else if (dt == DT_BF16) launch_k(k_nhwc_to_nchw<__nv_bfloat16>, grid, block, 0, s, (const __nv_bfloat16 *)x, y, C, HW);
     else if (dt == DT_F16) launch_k(k_nhwc_to_nchw<__half>, grid, block, 0, s, (const __half *)x, y, C, HW);

@@ -689,3 +689,23 @@ def test_int8_output_of_a_table_activation_bit_exact_at_every_scale_range(oracle
         assert np.array_equal(y, cur)
     finally:
         n.close()
+
+
+@pytest.mark.parametrize("precision", ["tf32", "f16"])
+@pytest.mark.parametrize("C,H,W", [(64, 1, 1), (68, 3, 11), (132, 5, 13), (260, 8, 8), (66, 4, 9)])
+def test_network_output_leaves_the_channels_last_layout(oracle_mod, precision, C, H, W):
+    """The re-layout of a network output: groups of four channels and ragged ones, pixels on both sides of a block of 32."""
+    from onenew_b200 import abi
+    from onenew_b200.one_file import OneBuilder
+    rng = np.random.default_rng(C + H * W)
+    w, bias = (rng.standard_normal((C, 16, 1, 1)) * 0.3).astype(np.float32), rng.standard_normal(C).astype(np.float32)
+    b = OneBuilder()
+    b.add_io("input", "input", (1, 16, H, W))
+    b.conv("Conv_0", "input", b.add_init("w", w), b.add_init("b", bias), "output", (1, 1), (1, 1), (0,) * 4, act=abi.NOT_ACT)
+    b.add_io("output", "output", (1, C, H, W))
+    x = rng.uniform(-1, 1, (3, 16, H, W)).astype(np.float32)
+    n = onet.Net(b.tobytes(), batch=3, precision=precision)
+    try:
+        assert_close(n(x), oracle_mod.conv_f32(x, w, bias, (1, 1), (0,) * 4, abi.NOT_ACT), f"{C}@{H}x{W}")
+    finally:
+        n.close()
