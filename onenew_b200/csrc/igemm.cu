@@ -282,7 +282,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     int qmode = 0;
     const uint8_t *qlut = sRes + 4;
     if constexpr (KIND == KIND_I8) {
-        if (p.tma_store == 2 && p.act == 3 && p.lut_smem && p.q_table) {
+        if (p.tma_store == 2 && p.act == 3 && p.lut_smem && p.q_table && p.consts) {
             const float h8 = __fmul_rn(8.f, p.q_inv_scale);
             if (h8 >= 126.5f && quant_s8(__ldg(p.lut + 8191), p.q_inv_scale) == 127) qmode = 1;
             else if (h8 >= 0.5f) qmode = 2;
@@ -297,11 +297,11 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             if (threadIdx.x == 0) sRes[3] = 0;
         }
     }
-    if (p.lut_smem && !qmode) {
-        static_assert(NEW * EPI_PATCH_BYTES >= 8192 * 4, "the table must fit the residual patches");
-        const float4 *g4 = reinterpret_cast<const float4 *>(p.lut);
+    static_assert(NEW * EPI_PATCH_BYTES >= 8192 * 4, "the table must fit the residual patches");
+    auto stage_table = [&](const float4 *g4) {
         for (int i = threadIdx.x; i < 2048; i += NUM_THREADS) reinterpret_cast<float4 *>(sRes)[i] = __ldg(g4 + i);
-    }
+    };
+    if (p.lut_smem && !qmode && p.consts) stage_table(reinterpret_cast<const float4 *>(p.lut));
     tc_fence_before_sync();
     // a pair: the peer's barriers and tensor memory must exist before anything of this CTA signals or writes them
     if constexpr (PAIR) cluster_sync();
@@ -318,6 +318,12 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     if (p.pdl) {
         pdl_launch_dependents();
         pdl_wait();
+    }
+    if (p.lut_smem && !p.consts) {   // the caller's table: an earlier kernel of the stream may have written it
+        const float4 *g4 = reinterpret_cast<const float4 *>(p.lut);
+        launder(g4);
+        stage_table(g4);
+        __syncthreads();
     }
 
     long long issued = 0;   // producer: ring stages whose loads were issued (ring position)

@@ -154,8 +154,10 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         tmem_alloc(smem_u32(tmem_slot), BN);
         tmem_relinquish();
     }
-    if (has_lut)   // a constant: staged before the wait
-        for (int i = threadIdx.x; i < 2048; i += THREADS) reinterpret_cast<float4 *>(slut)[i] = __ldg(reinterpret_cast<const float4 *>(p.lut) + i);
+    auto stage_table = [&](const float4 *g4) {
+        for (int i = threadIdx.x; i < 2048; i += THREADS) reinterpret_cast<float4 *>(slut)[i] = __ldg(g4 + i);
+    };
+    if (has_lut && u.b_const) stage_table(reinterpret_cast<const float4 *>(p.lut));
     tc_fence_before_sync();
     __syncthreads();
     if constexpr (S > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // (waited for before the first write to a peer)
@@ -259,7 +261,14 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     } else {
         if (p.pdl) pdl_wait();
     }
-    if (!u.b_const) load_constants();
+    if (!u.b_const) {   // the caller's tensors: an earlier kernel of the stream may have written them
+        load_constants();
+        if (has_lut) {
+            const float4 *g4 = reinterpret_cast<const float4 *>(p.lut);
+            launder(g4);
+            stage_table(g4);
+        }
+    }
     if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         const uint32_t idesc = make_idesc<KIND>(A_ROWS, BN) & ((KIND == KIND_BF16 && p.ab_f16) ? ~((7u << 7) | (7u << 10)) : ~0u);
@@ -402,6 +411,7 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
     }
     bool got = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0, abort_flag));
+    if (has_lut && !u.b_const) __syncthreads();   // every warp's part of the table is in place
     // Block w of the tile passes through shared memory (the ring is free: every MMA of the tile has completed) as 32 rows
     // of 128 bytes, 16-byte piece c of row x at c ^ (x & 7).  A cluster deals the rows out in S slices, CTA z finishes
     // slice z: each warp sends every slice of its partial block to its owner, [source CTA][block][row of the slice].

@@ -426,7 +426,7 @@ struct ConvIO {
     int coeff_finite;     // every int8 coefficient is finite
     float x_inv_scale;    // int8 + x_nchw_f32 explicit path: quantise while packing
     int y_nchw;           // y is fp32 in the reference layout
-    int w_const;          // w holds weights prepared before this call
+    int w_const;          // a prepared operator: w, bias, coeff and lut are its own copies, made before this call
 };
 
 // Store map for the epilogue's TMA path; *use is set to 1 when the output qualifies (no int8 copy, N a
@@ -542,6 +542,7 @@ int run_conv(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &
     p.lut_smem = p.act == SILU && p.lut && !p.residual && (reinterpret_cast<uintptr_t>(p.lut) & 15) == 0;
     p.out_q = io.out_q; p.q_inv_scale = io.q_inv_scale;
     p.q_table = pl.kind == KIND_I8 && io.coeff_finite && fabsf(e.in_scale) < 0x1p90f;
+    p.consts = io.w_const;
     p.status = ctx->status_dev;
     UnitParams u;
     memset(&u, 0, sizeof(u));
@@ -659,10 +660,11 @@ int run_gemm(one_ctx *ctx, int kind, const void *A, int a_pitch, const void *B, 
     p.bias_mode = bias ? BIAS_F32 : BIAS_NONE; p.bias = bias;
     if (epi) { p.act = epi->act; p.lut = epi->lut; p.residual = epi->residual; }
     p.lut_smem = p.act == SILU && p.lut && !p.residual && (reinterpret_cast<uintptr_t>(p.lut) & 15) == 0;
+    p.consts = tmB_cached != nullptr;   // (a cached map is a prepared operator's)
     p.status = ctx->status_dev;
     UnitParams u;
     memset(&u, 0, sizeof(u));
-    u.b_const = tmB_cached != nullptr;
+    u.b_const = p.consts;
     t_last_unit = (u.splits = choose_unit(auto_tile, M, N, batch, p.num_kb)) && unit_epilogue(kind, p, u) >= 0;
     if (tmB_cached && !t_last_unit) tmB = *tmB_cached;
     else {

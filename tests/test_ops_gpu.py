@@ -584,3 +584,35 @@ def test_chosen_tile_form_equals_plain_tiles(ops, oracle_mod, case):
         L.one_cuda_set_tile_n(0)
         L.one_cuda_set_eval_precision(capi.PREC_TF32)
     assert torch.equal(y, z) and bool(y.any())
+
+
+def _written_behind_a_long_kernel(pairs):
+    """Enqueue, on the legacy default stream, a kernel of some milliseconds and behind it this library's own copies
+    src -> dst (launched with the programmatic attribute, so that they let their successor start at once)."""
+    import ctypes as C
+    import torch
+    big = torch.ones((6144, 6144), device="cuda")
+    torch.cuda.synchronize()
+    big @ big
+    for src, dst in pairs:
+        n = C.c_longlong(src.numel())
+        capi.check(capi.lib().one_glue_copy_chunks(C.cast(src.data_ptr(), C.POINTER(C.c_float)), C.cast(dst.data_ptr(), C.POINTER(C.c_float)),
+                                                   C.c_longlong(1), n, C.c_longlong(1), n, n, None))
+
+
+# the one-wave kernel, its clusters along K, the persistent kernel with whole and ragged column chunks
+@pytest.mark.parametrize("shape", [(1, 64, 7, 7, 64), (1, 512, 7, 7, 70), (4, 32, 90, 90, 64), (4, 32, 90, 90, 33)], ids=["unit", "cluster", "tiles", "ragged_tiles"])
+def test_activation_table_written_just_before_the_call(ops, oracle_mod, shape):
+    """A drop-in Conv is ordered after the caller's earlier work, its activation table included."""
+    import torch
+    N, C, H, W, OC = shape
+    rng = np.random.default_rng(C + OC)
+    x = torch.from_numpy(rng.uniform(-1, 1, (N, C, H, W)).astype(np.float32)).cuda()
+    w = torch.from_numpy((rng.standard_normal((OC, C, 1, 1)) * 0.3).astype(np.float32)).cuda()
+    b = torch.from_numpy(rng.standard_normal(OC).astype(np.float32)).cuda()
+    table = torch.from_numpy(np.asarray(oracle_mod.silu_lut(), np.float32)).cuda()
+    want = ops.conv(x, w, b, act=abi.SILU, lut=table)
+    for _ in range(3):
+        lut = torch.full_like(table, 7.0)
+        _written_behind_a_long_kernel([(table, lut)])
+        assert torch.equal(ops.conv(x, w, b, act=abi.SILU, lut=lut), want)
