@@ -282,7 +282,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     int qmode = 0;
     const uint8_t *qlut = sRes + 4;
     if constexpr (KIND == KIND_I8) {
-        if (p.tma_store == 2 && p.act == 3 && p.lut_smem && p.q_table && p.consts) {
+        if (p.tma_store == 2 && p.act == 3 && p.lut_smem && p.q_table) {
             const float h8 = __fmul_rn(8.f, p.q_inv_scale);
             if (h8 >= 126.5f && quant_s8(__ldg(p.lut + 8191), p.q_inv_scale) == 127) qmode = 1;
             else if (h8 >= 0.5f) qmode = 2;
@@ -297,11 +297,11 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             if (threadIdx.x == 0) sRes[3] = 0;
         }
     }
-    static_assert(NEW * EPI_PATCH_BYTES >= 8192 * 4, "the table must fit the residual patches");
-    auto stage_table = [&](const float4 *g4) {
+    if (p.lut_smem && !qmode) {
+        static_assert(NEW * EPI_PATCH_BYTES >= 8192 * 4, "the table must fit the residual patches");
+        const float4 *g4 = reinterpret_cast<const float4 *>(p.lut);
         for (int i = threadIdx.x; i < 2048; i += NUM_THREADS) reinterpret_cast<float4 *>(sRes)[i] = __ldg(g4 + i);
-    };
-    if (p.lut_smem && !qmode && p.consts) stage_table(reinterpret_cast<const float4 *>(p.lut));
+    }
     tc_fence_before_sync();
     // a pair: the peer's barriers and tensor memory must exist before anything of this CTA signals or writes them
     if constexpr (PAIR) cluster_sync();
@@ -318,12 +318,6 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     if (p.pdl) {
         pdl_launch_dependents();
         pdl_wait();
-    }
-    if (p.lut_smem && !p.consts) {   // the caller's table: an earlier kernel of the stream may have written it
-        const float4 *g4 = reinterpret_cast<const float4 *>(p.lut);
-        launder(g4);
-        stage_table(g4);
-        __syncthreads();
     }
 
     long long issued = 0;   // producer: ring stages whose loads were issued (ring position)
@@ -1245,7 +1239,10 @@ static cudaError_t launch_one(const CUtensorMap &tmA, const CUtensorMap &tmB, co
     const long long sms = sm_count_of(dev);
     const long long slots = PAIR ? sms / 2 : sms;
     const unsigned grid = (unsigned)(tiles < slots ? tiles : slots) * (PAIR ? 2u : 1u);
-    p.pdl = get_pdl();
+    // A table that is the caller's may have been written by the launch before this one, and the kernel stages it before its
+    // wait: such a call is launched plainly.  (Staging it after the wait instead costs every other launch: the second copy
+    // of the loop and its barrier slowed the int8 backbone of 64 images from 1614 to 1649 us.)
+    p.pdl = get_pdl() && (p.consts || !p.lut_smem);
     p.epi_mode = g_epi_mode.load(std::memory_order_relaxed);
     cudaError_t e = launch_ex(igemm_kernel<KIND, BN, PAIR, MH, NEW>, dim3(grid), dim3(num_threads_for(NEW)), smem, stream, p.pdl != 0, PAIR ? 2 : 1, tmA, tmB, tmC, tmR, tmI, p);
     count_launch();
