@@ -315,6 +315,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     // accesses are ordered after it.  The next kernel may start its own prologue right away; it cannot
     // touch data before its own wait, which in turn covers this whole grid.
     // (The release of the next launch comes first: its blocks then do their own set-up while this one waits.)
+    // The epilogue's read-only loads (bias, coefficients, a table in global memory) stand behind the branch on the warp's
+    // role and the loop over tiles: a load that may not be executed is not moved up here, so their pointers need no laundering.
     if (p.pdl) {
         pdl_launch_dependents();
         pdl_wait();
@@ -1106,6 +1108,8 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const SplitKReducePa
         pdl_launch_dependents();
         pdl_wait();
     }
+    const float *partial = p.partial, *bias = p.bias, *lut = p.lut;
+    launder(partial); launder(bias); launder(lut);   // no load of theirs above the wait
     const bool out16 = out_is_16(p.out_mode), f16 = p.out_mode == OUT_F16;
     float vmax = 0.f;
     const long long quads_per_row = p.N >> 2;
@@ -1113,7 +1117,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const SplitKReducePa
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (long long)gridDim.x * blockDim.x) {
         const long long m = q / quads_per_row;
         const int n = (int)(q - m * quads_per_row) << 2;
-        const float *src = p.partial + m * p.partial_ld + n;
+        const float *src = partial + m * p.partial_ld + n;
         float4 acc = __ldcg(reinterpret_cast<const float4 *>(src));
         for (int z = 1; z < p.split_k; ++z) {
             const float4 t = __ldcg(reinterpret_cast<const float4 *>(src + (long long)z * p.plane_stride));
@@ -1121,16 +1125,16 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const SplitKReducePa
             acc.z = __fadd_rn(acc.z, t.z); acc.w = __fadd_rn(acc.w, t.w);
         }
         float v[4] = {acc.x, acc.y, acc.z, acc.w};
-        if (p.bias) {
+        if (bias) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = __fadd_rn(v[e], __ldg(p.bias + n + e));
+            for (int e = 0; e < 4; ++e) v[e] = __fadd_rn(v[e], __ldg(bias + n + e));
         }
         if (p.act == 1) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = v[e] > 0.f ? v[e] : 0.f;
         } else if (p.act != 0) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = apply_act(v[e], p.act, p.act_p0, p.act_p1, p.lut);
+            for (int e = 0; e < 4; ++e) v[e] = apply_act(v[e], p.act, p.act_p0, p.act_p1, lut);
         }
         const long long off = m * p.ldo + n;
         if (p.residual) {

@@ -176,12 +176,13 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const int col = n0 + c0 + chunk * 4, nvalid = p.N - col;        // this lane's four columns in a row-major output
     const bool f16 = p.out_mode == OUT_F16;
     alignas(16) float cst_[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const float *gbias = reinterpret_cast<const float *>(p.bias), *gcoeff = p.coeff;
     auto load_constants = [&]() {
         if (ROWS && nvalid > 0) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                if (p.bias) cst_[e] = __ldg(reinterpret_cast<const float *>(p.bias) + col + e);
-                if (KIND == KIND_I8) cst_[4 + e] = __ldg(p.coeff + col + e);
+                if (gbias) cst_[e] = __ldg(gbias + col + e);
+                if (KIND == KIND_I8) cst_[4 + e] = __ldg(gcoeff + col + e);
             }
         }
     };
@@ -261,7 +262,10 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     } else {
         if (p.pdl) pdl_wait();
     }
-    if (!u.b_const) {   // the caller's tensors: an earlier kernel of the stream may have written them
+    // The caller's tensors, which an earlier kernel of the stream may have written: read through laundered pointers, so that
+    // no read-only load of theirs can be moved above the wait (or merged with one that stands there).
+    launder(gbias); launder(gcoeff);
+    if (!u.b_const) {
         load_constants();
         if (has_lut) {
             const float4 *g4 = reinterpret_cast<const float4 *>(p.lut);
@@ -307,6 +311,8 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             // 16-byte pieces of the K-major tiles: piece c of row r lies at c ^ (r & 7) within a 128-byte row (narrower
             // rows: the corresponding swizzle), so an in-place pass needs no addresses but the linear ones.
             const int t = threadIdx.x - 64;
+            const float *ga = u.a, *gb = u.b;
+            launder(ga); launder(gb);
             auto rnd4 = [](uint4 v) {
                 return make_uint4(__float_as_uint(round_to_tf32(__uint_as_float(v.x))), __float_as_uint(round_to_tf32(__uint_as_float(v.y))),
                                   __float_as_uint(round_to_tf32(__uint_as_float(v.z))), __float_as_uint(round_to_tf32(__uint_as_float(v.w))));
@@ -332,7 +338,7 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 c = u.b_ld == 2 ? j / BN : j & (cpr - 1);
             };
             auto fetch_b = [&](int i) {
-                const float *base = u.b + (long long)bz * u.b_bstride;
+                const float *base = gb + (long long)bz * u.b_bstride;
 #pragma unroll
                 for (int q = 0; q < BPIECES; ++q) {
                     int r, c;
@@ -347,7 +353,7 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 const int k0 = (kb0 + i) * p.slab_elems;
                 if ((u.a_ld || u.b_ld) && i >= stages && !mbar_wait(empty0 + 8 * s, phase ^ 1, abort_flag)) ok = false;
                 if (ok && u.a_ld) {
-                    const float *base = u.a + (long long)bz * u.a_bstride;
+                    const float *base = ga + (long long)bz * u.a_bstride;
 #pragma unroll 3
                     for (int j = t; j < A_ROWS * cpr; j += 192) {
                         const int r = j >> cshift, c = j & (cpr - 1);
@@ -536,7 +542,7 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 #pragma unroll
                 for (int z = 1; z < S; ++z) raw[0] = add_partial<KIND>(raw[0], *reinterpret_cast<const uint32_t *>(src + z * (NBLK * PER * 128)));
                 if (m >= p.M || n >= p.N) continue;
-                const float b[1] = {p.bias ? __ldg(reinterpret_cast<const float *>(p.bias) + n) : 0.f}, k[1] = {KIND == KIND_I8 ? __ldg(p.coeff + n) : 0.f};
+                const float b[1] = {gbias ? __ldg(gbias + n) : 0.f}, k[1] = {KIND == KIND_I8 ? __ldg(gcoeff + n) : 0.f};
                 float t[1];
                 finish<KIND, 1>(t, raw, b, k, p, slut);
                 long long off;

@@ -616,3 +616,20 @@ def test_activation_table_written_just_before_the_call(ops, oracle_mod, shape):
         lut = torch.full_like(table, 7.0)
         _written_behind_a_long_kernel([(table, lut)])
         assert torch.equal(ops.conv(x, w, b, act=abi.SILU, lut=lut), want)
+
+
+@pytest.mark.parametrize("M,K,N", [(64, 256, 64), (33, 1027, 70), (900, 512, 1600)])
+def test_operands_written_just_before_the_call(ops, M, K, N):
+    """The same for operands read where they lie (by TMA, by plain loads, and packed first) and for the bias."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+    a, w, b = (torch.randn(s, generator=gen, device="cuda") for s in ((M, K), (N, K), (N,)))
+    kn = w.t().contiguous()
+    x, cw = torch.randn((2, 64, 9, 11), generator=gen, device="cuda"), torch.randn((N, 64, 3, 3), generator=gen, device="cuda")
+    calls = [(ops.gemm, (a, w, b)), (ops.matmul, (a, kn)), (ops.conv, (x, cw, b))]   # K-major by TMA or plain loads, [K][N], packed
+    for fn, args in calls:
+        want = fn(*args)
+        for _ in range(2):
+            late = [torch.full_like(t, 3.0) for t in args]
+            _written_behind_a_long_kernel(list(zip(args, late)))
+            assert torch.equal(fn(*late), want), fn.__name__
