@@ -721,16 +721,49 @@ void dequant_coeffs(const CONV_CONFIG_S *cfg, int OC, std::vector<float> *out)
     for (int i = 0; i < OC; ++i) (*out)[i] = cfg->weight_aux[i] * 1 / 127.0f;
 }
 
+// Whether two ranges of device memory share a byte.
+inline bool overlap(const void *a, size_t a_bytes, const void *b, size_t b_bytes)
+{
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + b_bytes && y < x + a_bytes;
+}
+
+// A convolution whose output is the reference layout, written by the epilogue itself -- or, when `out` shares memory with a
+// tensor that the launch reads (an earlier CTA's output would be another's bias or table), through an NHWC copy in the workspace.
+// Input and weights have been copied into the workspace by then.
+int run_conv_nchw(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &pl, ConvIO io, const CUtensorMap *tmB_cached,
+                  float *out, cudaStream_t stream)
+{
+    const long long M = (long long)g.N * g.OH * g.OW;
+    const size_t out_bytes = (size_t)M * g.OC * 4;
+    io.out_mode = OUT_F32;
+    if ((io.bias && overlap(out, out_bytes, io.bias, (size_t)g.OC * 4)) || (e.act == SILU && overlap(out, out_bytes, io.lut, 8192 * 4))) {
+        void *yh = ws_alloc(ctx, out_bytes);
+        if (!yh) return fail(ONE_ERR_NOMEM, "Conv: workspace too small for the NHWC output");
+        io.y = yh;
+        int rc = run_conv(ctx, g, e, pl, io, tmB_cached, stream);
+        if (rc != ONE_OK) return rc;
+        cudaError_t ce = nhwc_to_nchw(yh, out, g.N, g.OC, g.OH * g.OW, DT_F32, stream);
+        return ce == cudaSuccess ? ONE_OK : cuda_fail(ce, "nhwc_to_nchw");
+    }
+    io.y = out;
+    io.y_nchw = 1;
+    return run_conv(ctx, g, e, pl, io, tmB_cached, stream);
+}
+
 // A one-wave fp32 product of caller tensors with tf32 operands, read where they lie: D = A * B^T with A [batch][M][K] and B
 // [batch][N][K], or [batch][K][N] (`b_kn`).  Rows of whole 16-byte pieces come by TMA; others, and a [K][N] operand, by plain
 // loads, which keep up only over a short K range: at most RAW_PLAIN_KB blocks a CTA.  Saves the packing kernels, their launches
 // and their passes over memory: Gemm 256 x 2048 x 1000 37.1 -> 35.8 us a call, MatMul 24 x 197 x 64 x 197 30.7 -> 29.5.
-// Returns ONE_OK, an error, or 1 when the call is not of this form (the caller packs the operands).
+// Returns ONE_OK, an error, or 1 when the call is not of this form (the caller packs the operands): an output that shares memory
+// with an operand is not, since some CTAs still read what others have overwritten.
 constexpr int RAW_PLAIN_KB = 8;
 int run_raw(one_ctx *ctx, int kind, const float *A, const float *B, int b_kn, long long M, int N, int K, int batch, float *out, const float *bias,
             cudaStream_t stream)
 {
     if (kind != KIND_TF32 || M > 0x7fffffffLL) return 1;
+    const size_t nb = batch ? (size_t)batch : 1, out_bytes = nb * M * N * 4;
+    if (overlap(out, out_bytes, A, nb * M * K * 4) || overlap(out, out_bytes, B, nb * N * K * 4)) return 1;
     const int slab_bytes = slab_for_bytes((long long)K * 4), num_kb = (int)(((long long)K * 4 + slab_bytes - 1) / slab_bytes);
     UnitParams u;
     memset(&u, 0, sizeof(u));
@@ -774,7 +807,8 @@ size_t conv_eval_scratch(const ConvGeom &g, const ConvEpi &e, const ConvPlan &pl
     else if (pl.path == PATH_S2D) need += up256((size_t)g.N * pl.Hs * pl.Ws * pl.Cp * pl.es);
     else need += up256((size_t)g.N * g.H * g.W * g.C * pl.es);
     need += up256((size_t)g.OC * pl.w_pitch * pl.es);
-    need += up256((size_t)M * g.OC * 4);   // (an NHWC copy of the output, no longer made: the same shapes are refused as before)
+    need += up256((size_t)M * g.OC * 4);   // the NHWC copy of the output: counted whether or not run_conv_nchw makes it, so that
+                                           // what fits does not depend on where the caller's tensors lie
     if (e.int8) need += 2 * up256((size_t)g.OC * 4);
     return need;
 }
@@ -942,10 +976,7 @@ extern "C" int one_cuda_conv_eval(BUFFER_INFO_S *params, BUFFER_INFO_S *inputs, 
             return cuda_fail(ce, "coefficient upload");
         io.coeff = cd;
     }
-    io.y = reinterpret_cast<void *>(outputs[0].addr);   // the epilogue writes the reference layout itself
-    io.y_nchw = 1;
-    io.out_mode = OUT_F32;
-    if ((rc = run_conv(ctx, g, e, pl, io, nullptr, st)) != ONE_OK) return rc;
+    if ((rc = run_conv_nchw(ctx, g, e, pl, io, nullptr, reinterpret_cast<float *>(outputs[0].addr), st)) != ONE_OK) return rc;
     return finish_sync(ctx, st);
 }
 
@@ -1337,8 +1368,7 @@ extern "C" int one_cuda_eval_async(one_ctx *ctx, one_packed *op, BUFFER_INFO_S *
                     return cuda_fail(ce, "nchw_to_nhwc");
                 io.x = xh;
             }
-            io.y = reinterpret_cast<void *>(outputs[0].addr); io.y_nchw = 1; io.out_mode = OUT_F32;
-            if ((rc = run_conv(ctx, g, op->e, op->pl, io, &op->tmB, st)) != ONE_OK) return rc;
+            if ((rc = run_conv_nchw(ctx, g, op->e, op->pl, io, &op->tmB, reinterpret_cast<float *>(outputs[0].addr), st)) != ONE_OK) return rc;
         } else {
             // device-resident NHWC activations
             if (op->flags & ONE_IN_NCHW_F32) {
@@ -1552,9 +1582,6 @@ extern "C" int one_cuda_conv_eval_static(BUFFER_INFO_S *params, BUFFER_INFO_S *i
         io.coeff = cd;
     }
     io.lut = reinterpret_cast<const float *>(inputs[BUF_MAXNUM - 1].addr);
-    io.y = reinterpret_cast<void *>(outputs[0].addr);
-    io.y_nchw = 1;
-    io.out_mode = OUT_F32;
-    if ((rc = run_conv(ctx, g, e, pl, io, nullptr, st)) != ONE_OK) return rc;
+    if ((rc = run_conv_nchw(ctx, g, e, pl, io, nullptr, reinterpret_cast<float *>(outputs[0].addr), st)) != ONE_OK) return rc;
     return finish_sync(ctx, st);   // waits for the stream; `coeff` above stays alive until then
 }

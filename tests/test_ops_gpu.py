@@ -633,3 +633,52 @@ def test_operands_written_just_before_the_call(ops, M, K, N):
             late = [torch.full_like(t, 3.0) for t in args]
             _written_behind_a_long_kernel(list(zip(args, late)))
             assert torch.equal(fn(*late), want), fn.__name__
+
+
+def test_output_that_shares_memory_with_an_input(ops):
+    """Gemm and MatMul take copies of operands that the output overlaps, Conv of its bias and table too (the input and the
+    weights always): the results are those of separate tensors.  A MatMul's A of whole 16-byte rows is read in place by every
+    path and is not among them."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    def rand(*s):
+        return torch.randn(s, generator=gen, device="cuda")
+    for n in (260, 131):
+        a, w, b = rand(n, n), rand(n, n), rand(n)
+        want = ops.gemm(a, w, b)
+        for which in range(3):
+            pool = torch.zeros(4 * n * n + 64, device="cuda")
+            slots = [pool[i * n * n:(i + 1) * n * n] for i in range(2)]
+            slots[0].copy_(a.ravel()); slots[1].copy_(w.ravel())
+            # onto A, onto W, or across the end of W
+            y = slots[which] if which < 2 else pool[2 * n * n - 36:3 * n * n - 36]
+            args = abi.gemm_eval_args((n, n), (n, n), (n, n), slots[0].data_ptr(), slots[1].data_ptr(), b.data_ptr(), y.data_ptr())
+            capi.check(capi.shim_eval("Gemm")(args.params, args.inputs, args.outputs))
+            # (packed operands are rounded as the ones read in place are: only the order of the sums differs)
+            assert (y.view(n, n) - want).norm() <= 1e-5 * want.norm(), (n, which)
+        want = ops.matmul(a, w)
+        for onto_b in ([True] if n % 4 == 0 else [True, False]):
+            ca, cw = a.clone(), w.clone()
+            y = cw if onto_b else ca
+            args = abi.matmul_eval_args((n, n), (n, n), (n, n), ca.data_ptr(), cw.data_ptr(), y.data_ptr())
+            capi.check(capi.shim_eval("MatMul")(args.params, args.inputs, args.outputs))
+            # A in place is cut to tf32 by the tensor core instead of rounded: up to 2^-10 a product
+            assert (y - want).norm() <= (1e-3 if n % 4 == 0 else 1e-5) * want.norm(), (n, onto_b)
+    from onenew_b200 import net
+    table = torch.from_numpy(net.activation_table("silu")).cuda()
+    for N, Cc, hw, OC in ((2, 64, 9, 64), (2, 32, 120, 96), (1, 32, 20, 30)):
+        x, w, b = rand(N, Cc, hw, hw), rand(OC, Cc, 3, 3) * 0.05, rand(OC)
+        want = ops.conv(x, w, b, pads=(1,) * 4, act=abi.SILU, lut=table)
+        # the table, or the bias, in the middle of the output
+        pool = torch.zeros(want.numel() + 8192 + 64, device="cuda")
+        cfg = abi.conv_cfg((3, 3), (1, 1), (1,) * 4, has_bias=True, act=abi.SILU)
+        for name in ("table", "bias"):
+            at = 4 * (want.numel() // 8)
+            src = table if name == "table" else b
+            inside = pool[at:at + src.numel()]
+            inside.copy_(src)
+            args = abi.conv_eval_args(cfg, tuple(x.shape), tuple(w.shape), tuple(want.shape), x.data_ptr(), w.data_ptr(),
+                                      inside.data_ptr() if name == "bias" else b.data_ptr(), pool.data_ptr(), abi.default_useful_info(),
+                                      inside.data_ptr() if name == "table" else table.data_ptr())
+            capi.check(capi.shim_eval("Conv")(args.params, args.inputs, args.outputs))
+            assert torch.equal(pool[:want.numel()].view_as(want), want), (OC, name)
