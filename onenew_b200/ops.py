@@ -6,8 +6,9 @@ only) and calls the ``eval`` symbol of the drop-in library ``lib<Op>_cu.so``.  S
 layouts are the reference's: NCHW fp32 activations, OIHW weights, [N][K] Gemm weights.
 
 The descriptors a call passes depend on its shapes and options alone, so a bounded table keeps the
-``params`` array of each combination (building the ctypes records anew took a fifth of a small call);
-the libraries only read them.  Pointers are written into fresh ``inputs`` / ``outputs`` arrays per call.
+``params`` array of each combination of whole numbers (building the ctypes records anew took a fifth of a
+small call); the libraries only read them.  Other options (a clip range, a slope: floats, lists, arrays) are
+written anew each time.  Pointers go into fresh ``inputs`` / ``outputs`` arrays per call.
 """
 import functools
 
@@ -32,13 +33,21 @@ def out_hw(H, W, KH, KW, strides, pads):
     return ((H + pads[0] + pads[2] - KH) // strides[1] + 1, (W + pads[1] + pads[3] - KW) // strides[0] + 1)
 
 
-@functools.lru_cache(maxsize=256)
-def _conv_plan(x_shape, w_shape, strides, pads, has_bias, act, cfg_items):
-    """(output shape, params holder) of one conv shape; fp32 only (an int8 config carries its scales)."""
+def _conv_args(x_shape, w_shape, strides, pads, has_bias, act, **cfg_kw):
+    """(output shape, params holder) of one conv."""
     N, _, H, W = x_shape
-    y_shape = (N, w_shape[0]) + out_hw(H, W, w_shape[2], w_shape[3], strides, pads)
-    cfg = abi.conv_cfg(w_shape[2:], strides, pads, has_bias=has_bias, act=act, **dict(cfg_items))
+    OC, _, KH, KW = w_shape
+    y_shape = (N, OC) + out_hw(H, W, KH, KW, strides, pads)
+    cfg = abi.conv_cfg((KH, KW), strides, pads, has_bias=has_bias, act=act, **cfg_kw)
     return y_shape, abi.conv_eval_args(cfg, x_shape, w_shape, y_shape, 0, 0, 0, 0, abi.default_useful_info())
+
+
+_conv_plan = functools.lru_cache(maxsize=256)(_conv_args)
+
+
+def _whole(values):
+    """Plain whole numbers only: equal keys then write equal records (2.0 == 2, True == 1 and -0.0 == 0.0 would not)."""
+    return all(type(v) is int for v in values)
 
 
 @functools.lru_cache(maxsize=256)
@@ -76,20 +85,17 @@ def conv(x, w, b, strides=(1, 1), pads=(0, 0, 0, 0), act=abi.NOT_ACT, int8=None,
     if int8 is None:
         wd = _dev(w)   # depthwise: pass group=C in cfg_kw, weight [C][1][KH][KW]
         bd = _dev(b) if b is not None else None
-        y_shape, plan = _conv_plan(tuple(xd.shape), tuple(wd.shape), tuple(strides), tuple(pads), b is not None, act, tuple(sorted(cfg_kw.items())))
+        strides, pads = tuple(strides), tuple(pads)
+        plan_of = _conv_plan if _whole((*strides, *pads, act, *cfg_kw.values())) else _conv_args
+        y_shape, plan = plan_of(tuple(xd.shape), tuple(wd.shape), strides, pads, b is not None, act, **cfg_kw)
         return _call("Conv", plan, y_shape, xd, wd, bd, lutd)
-    N, Cc, H, W = xd.shape
-    OC, _, KH, KW = w.shape
-    OH, OW = out_hw(H, W, KH, KW, strides, pads)
     wd = torch.zeros(int(np.prod(w.shape)), dtype=torch.float32, device="cuda")
     wd.view(torch.int8)[: wd.numel()] = _dev(np.asarray(w, np.int8).ravel(), torch.int8)
     bd = None
     if b is not None:
         bd = _dev(np.asarray(b, np.int32), torch.int32)
-    cfg = abi.conv_cfg((KH, KW), strides, pads, has_bias=b is not None, act=act, int8_scale=int8[0],
-                       weight_aux=int8[1], **cfg_kw)
-    plan = abi.conv_eval_args(cfg, (N, Cc, H, W), tuple(w.shape), (N, OC, OH, OW), 0, 0, 0, 0, abi.default_useful_info())
-    return _call("Conv", plan, (N, OC, OH, OW), xd, wd, bd, lutd)
+    y_shape, plan = _conv_args(tuple(xd.shape), tuple(w.shape), strides, pads, b is not None, act, int8_scale=int8[0], weight_aux=int8[1], **cfg_kw)
+    return _call("Conv", plan, y_shape, xd, wd, bd, lutd)
 
 
 def gemm(a, w, b):

@@ -83,3 +83,23 @@ def test_bad_descriptors_are_rejected_before_any_launch():
     assert L.one_cuda_conv_eval(a.params, a.inputs, a.outputs) == -1
     m = abi.matmul_eval_args((2, 4, 8), (3, 8, 5), (2, 4, 5), 16, 16, 16)
     assert L.one_cuda_matmul_eval(m.params, m.inputs, m.outputs) == -2
+
+
+def test_operator_options_of_any_form(monkeypatch):
+    """``ops.conv`` keeps the records of a combination of whole numbers; other options, hashable or not, are written as they are."""
+    import numpy as np
+    import torch
+    from onenew_b200 import ops
+    monkeypatch.setattr(ops, "_dev", lambda a, dtype=torch.float32: torch.as_tensor(a, dtype=dtype))
+    monkeypatch.setattr(ops, "_call", lambda op, plan, y_shape, *tensors: abi.CONV_CONFIG_S.from_address(plan.params[0].addr))
+    x, w, b = np.zeros((1, 3, 8, 8), np.float32), np.zeros((4, 3, 3, 3), np.float32), np.zeros(4, np.float32)
+    for clip in ([0.5, 6.0], (0.5, 6.0), np.array([0.5, 6.0])):
+        cfg = ops.conv(x, w, b, act=abi.CLIP, clip=clip)
+        assert (cfg.clip_min, cfg.clip_max) == (0.5, 6.0)
+    assert np.copysign(1, ops.conv(x, w, b, act=abi.CLIP, clip=(0.0, 6.0)).clip_min) == 1
+    assert np.copysign(1, ops.conv(x, w, b, act=abi.CLIP, clip=(-0.0, 6.0)).clip_min) == -1
+    for strides in ([2, 2], (2, 2)):
+        assert list(ops.conv(x, w, b, strides=strides, pads=[1, 1, 1, 1]).strides)[:2] == [2, 2]
+    with pytest.raises(TypeError):          # refused by the record's integer field, whatever has been kept before
+        ops.conv(x, w, b, strides=(2.0, 2.0), pads=[1, 1, 1, 1])
+    assert ops.conv(x[:, :1], w[:1, :1], None, group=1).has_bias == 0
