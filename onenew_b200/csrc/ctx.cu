@@ -7,7 +7,6 @@
 #include <atomic>
 #include <map>
 #include <mutex>
-#include <vector>
 
 #include "../../include/one_cuda.h"
 
@@ -52,56 +51,45 @@ void *ws_alloc(one_ctx *c, size_t bytes)
     return c->ws + off;
 }
 
-// Status words are slots of mapped pages that live as long as the process (pinning a page takes ~10 ms, too long for
-// every context); a context gives its slot back when it is released, and another page is pinned only when all are taken.
-struct StatusPage {
-    static constexpr size_t SLOTS = 1024;
-    unsigned int *words = nullptr;
-    bool used[SLOTS] = {};
-};
-static std::mutex g_slot_mu;
-static std::vector<StatusPage *> g_status_pages;
-
-static cudaError_t status_slot_take(unsigned int **host, unsigned int **dev)
-{
-    std::lock_guard<std::mutex> lk(g_slot_mu);
-    for (size_t page = 0;; ++page) {
-        if (page == g_status_pages.size()) {
-            void *p = nullptr;
-            cudaError_t e = cudaHostAlloc(&p, StatusPage::SLOTS * sizeof(unsigned int), cudaHostAllocMapped | cudaHostAllocPortable);
-            if (e != cudaSuccess) return e;
-            g_status_pages.push_back(new StatusPage);
-            g_status_pages.back()->words = static_cast<unsigned int *>(p);
-        }
-        StatusPage *pg = g_status_pages[page];
-        for (size_t i = 0; i < StatusPage::SLOTS; ++i) {
-            if (pg->used[i]) continue;
-            void *d = nullptr;
-            cudaError_t e = cudaHostGetDevicePointer(&d, pg->words + i, 0);
-            if (e != cudaSuccess) return e;
-            pg->used[i] = true;
-            pg->words[i] = 0;
-            *host = pg->words + i;
-            *dev = static_cast<unsigned int *>(d);
-            return cudaSuccess;
-        }
+// Status words (see status_pages.h).
+namespace {
+typedef CUresult (*PFN_ctxGetCurrent)(CUcontext *);
+typedef CUresult (*PFN_ctxGetId)(CUcontext, unsigned long long *);
+struct CudaPages {
+    static int id(unsigned long long *out)
+    {
+        static PFN_ctxGetCurrent current = nullptr;
+        static PFN_ctxGetId get_id = nullptr;
+        static std::once_flag once;
+        std::call_once(once, [] {
+            cudaDriverEntryPointQueryResult q;
+            void *fn = nullptr;
+            if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &fn, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+                current = reinterpret_cast<PFN_ctxGetCurrent>(fn);
+            fn = nullptr;
+            if (cudaGetDriverEntryPoint("cuCtxGetId", &fn, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+                get_id = reinterpret_cast<PFN_ctxGetId>(fn);
+        });
+        CUcontext c = nullptr;
+        if (!current || !get_id) return cudaErrorNotSupported;
+        if (current(&c) != CUDA_SUCCESS || !c || get_id(c, out) != CUDA_SUCCESS) return cudaErrorDeviceUninitialized;
+        return 0;
     }
-}
-
-static void status_slot_give(const volatile unsigned int *host)
-{
-    if (!host) return;
-    std::lock_guard<std::mutex> lk(g_slot_mu);
-    for (StatusPage *pg : g_status_pages)
-        if (host >= pg->words && host < pg->words + StatusPage::SLOTS) pg->used[host - pg->words] = false;
-}
+    static int pin(unsigned int **p, size_t words) { return cudaHostAlloc(reinterpret_cast<void **>(p), words * sizeof(unsigned int), cudaHostAllocMapped); }
+    static int unpin(unsigned int *p) { return cudaFreeHost(p); }
+    static int map(unsigned int **dev, unsigned int *host) { return cudaHostGetDevicePointer(reinterpret_cast<void **>(dev), host, 0); }
+};
+// never destroyed: contexts may be released while the process ends
+StatusPages<CudaPages> &status_pages() { static auto *p = new StatusPages<CudaPages>; return *p; }
+}  // namespace
 
 int take_status(one_ctx *c)
 {
     unsigned int st = 0;
-    if (c->status_host) {
-        st = *c->status_host;
-        if (st) *c->status_host = 0;
+    if (c->status.host) {
+        volatile unsigned int *word = c->status.host;
+        st = *word;
+        if (st) *word = 0;
     } else {
         cudaError_t e = cudaMemcpy(&st, c->status_dev, sizeof(st), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(e, "status read");
@@ -248,23 +236,22 @@ extern "C" int one_cuda_init(int device, size_t workspace_bytes, one_ctx **out)
         return fail(ONE_ERR_UNSUPPORTED, "device %d is sm_%d%d; this library holds sm_100a code only", device,
                     prop.major, prop.minor);
     one_ctx *c = new one_ctx();
-    unsigned int *status_host = nullptr;
     c->device = device;
     c->ws_bytes = workspace_bytes ? workspace_bytes : (size_t(256) << 20);
     if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaMalloc(&c->ws, c->ws_bytes)) != cudaSuccess ||
-        (e = status_slot_take(&status_host, &c->status_dev)) != cudaSuccess ||
+        (e = static_cast<cudaError_t>(status_pages().take(device, &c->status))) != cudaSuccess ||
         (e = cudaMalloc(&c->ident16[0], 2 * 64 * 64 * 2)) != cudaSuccess) {
         int rc = cuda_fail(e, "one_cuda_init allocation");
         if (c->ws) cudaFree(c->ws);
-        status_slot_give(status_host);
+        status_pages().give(&c->status);
         if (c->ident16[0]) cudaFree(c->ident16[0]);
         if (c->stream) cudaStreamDestroy(c->stream);
         delete c;
         cudaSetDevice(prev);
         return rc;
     }
-    c->status_host = status_host;
+    c->status_dev = c->status.dev;
     {   // 1.0 on the diagonal: 0x3F80 in bf16, 0x3C00 in fp16
         static uint16_t host[2][64 * 64];
         for (int f = 0; f < 2; ++f)
@@ -288,7 +275,7 @@ extern "C" int one_cuda_release(one_ctx *c)
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     cudaFree(c->ws);
-    status_slot_give(c->status_host);
+    status_pages().give(&c->status);
     cudaFree(c->ident16[0]);
     cudaStreamDestroy(c->stream);
     delete c;

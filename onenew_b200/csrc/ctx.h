@@ -9,6 +9,8 @@
 
 #include <string>
 
+#include "status_pages.h"
+
 struct one_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -17,9 +19,9 @@ struct one_ctx {
     size_t ws_off = 0;          // bump offset of the call in progress
     // Status word the kernels report through: pinned host memory mapped into the device's address space, so that the
     // host reads it after a stream synchronisation without a copy (~8 us of every synchronous call).  A context whose
-    // word lives in device memory (the allocation-free Conv) has no host view of it: status_host is null then.
+    // word lives in device memory (the allocation-free Conv) has no host view of it: status.host is null then.
     unsigned int *status_dev = nullptr;
-    volatile unsigned int *status_host = nullptr;
+    one::StatusSlot status;
     bool allow_split = true;    // split-K contractions may take scratch for their partial sums
     void *ident16[2] = {nullptr, nullptr};   // 64 x 64 identity matrices in bf16 [0] and fp16 [1] (residual added by the tensor core)
 };

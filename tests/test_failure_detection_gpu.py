@@ -1,5 +1,9 @@
 """Failure detection without a GPU fault: a device-side wait that runs out is reported through the
 status word as ONE_ERR_TIMEOUT, the kernel returns normally and the context keeps working."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -42,3 +46,30 @@ def test_host_side_injection_is_rejected_before_launch():
     a = abi.conv_eval_args(cfg, (1, 8, 8, 8), (8, 8, 3, 3), (1, 8, 9, 8), 16, 16, 16, 16, u)
     assert L.one_cuda_conv_eval(a.params, a.inputs, a.outputs) == -2
     assert L.one_cuda_launch_count() == before
+
+
+RESET = """
+import ctypes, glob, os, torch
+from onenew_b200 import capi
+rt = ctypes.CDLL(glob.glob(os.path.join(os.path.dirname(torch.__file__), "..", "nvidia", "cuda_runtime", "lib", "libcudart.so.12"))[0])
+for released in (True, False, True):
+    ctx = capi.Context(0, 1 << 24)
+    ctx.status()
+    capi.check(capi.lib().one_cuda_selftest_wait_timeout(ctx.handle, 1 << 16))
+    try:
+        ctx.status()
+        raise SystemExit("the wait was not reported")
+    except capi.OneCudaError as e:
+        assert e.code == -6
+    ctx.status()
+    if released:
+        ctx.close()
+    ctx.handle = None
+    assert rt.cudaDeviceReset() == 0
+"""
+
+
+def test_a_new_context_after_the_host_reset_its_device():
+    """Nothing that outlives a context is read after cudaDeviceReset (which ends this process's own context only)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", RESET], cwd=root, check=True, timeout=300)
