@@ -152,6 +152,9 @@ ONE_API int one_cuda_packed_work(one_packed *op, double *flops, double *bytes);
 /* Text describing the last evaluation of a prepared operator (GEMM view M, N, K, operand type, output
  * tile, split-K ranges) for per-operator performance tables. */
 ONE_API int one_cuda_packed_detail(one_packed *op, char *buf, size_t cap);
+/* The output tile, split-K ranges and form of the calling thread's last contraction, drop-in calls included:
+ * "tile=128x64 split=4 unit" (one tile per CTA), or "2cta" / "2half" / "12w" for the tile codes below. */
+ONE_API int one_cuda_last_form(char *buf, size_t cap);
 /* Failure-detection self test.  Enqueues, on the context's stream, a one-warp kernel that waits on a
  * barrier nothing ever completes, gives up after `limit_clocks` GPU clocks (at most 2^31) and records
  * that in the status word the way a stalled pipeline role of the contraction kernel would.  The next
@@ -170,7 +173,8 @@ ONE_API int one_cuda_set_tile_n(int bn);
  * tiles would occupy at most half the SMs cuts its K range into several pieces, each piece accumulated
  * by its own CTA into a scratch plane, the planes added in a fixed order by a second short kernel that
  * also applies bias / activation / residual), 1 = never split, 2..64 = that many pieces when the shape
- * allows it.  Only the float paths split that way; results do not depend on scheduling.  With 0, and no tile
+ * allows it (output rows and bias of whole 16-byte pieces, scratch for the planes, and no tile code above 1000
+ * asked for).  Only the float paths split that way; results do not depend on scheduling.  With 0, and no tile
  * override, a launch whose 128 x 64 tiles are all resident at once runs one tile per CTA instead, its K range
  * shared by a cluster of up to eight CTAs; 1 therefore also gives sums that do not depend on the batch. */
 ONE_API int one_cuda_set_split_k(int splits);

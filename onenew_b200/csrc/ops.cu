@@ -41,8 +41,14 @@ static std::atomic<int> g_cta_pairs{1};   // tile codes 1xxx (pairs of CTAs) are
 static std::atomic<int> g_half_tiles{1};  // tile codes 2xxx (two 128-row halves per CTA) are accepted
 static std::atomic<int> g_wide_epi{1};    // tile codes 4xxx (twelve epilogue warps) are accepted
 thread_local int t_pairing = 1;      // width pairing of narrow multi-tap convolutions (see pair_geometry)
-thread_local int t_last_split = 1;   // K ranges the last contraction enqueued by this thread was cut into
-thread_local int t_last_unit = 0;    // whether it took the unit kernel
+// Form of the last contraction enqueued by this thread: tile width, K ranges, and how the tiles are walked.
+struct LastForm {
+    int bn = 0, split = 1;
+    const char *how = "";
+};
+thread_local LastForm t_last;
+inline void note_form(int bn, int split, const char *how) { t_last.bn = bn; t_last.split = split; t_last.how = how; }
+inline const char *form_name(bool cta2, int mh, int nw) { return cta2 ? " 2cta" : (mh == 2 ? " 2half" : (nw == 12 ? " 12w" : "")); }
 thread_local int t_split_k = 0;   // 0: the library's choice, 1: never split, n > 1: force n ranges (clamped to the K blocks)
 
 struct ConvGeom {
@@ -473,10 +479,18 @@ inline bool vec_constants_ok(const IgemmParams &p)
     return ((reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.coeff)) & 15) == 0;
 }
 
-// Enqueue one convolution.  `amap` (optional) caches the A tensor map between calls.
-int run_conv(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &pl, const ConvIO &io,
+// A forced number of K ranges wants plain tiles: pairs and halves, where they are the library's own choice, give way.
+inline bool plain_for_split(int auto_tile, int kind) { return t_split_k > 1 && auto_tile && kind != KIND_I8; }
+
+// Enqueue one convolution.  `tmB_cached` (optional): the B tensor map, kept between calls.
+int run_conv(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &plan, const ConvIO &io,
              const CUtensorMap *tmB_cached, cudaStream_t stream)
 {
+    ConvPlan pl = plan;
+    if (plain_for_split(pl.auto_tile, pl.kind)) {
+        if (pl.cta2) tmB_cached = nullptr;   // its box is half a tile
+        pl.cta2 = 0; pl.mh = 1; pl.nw = 8;
+    }
     const long long M = (long long)g.N * g.OH * g.OW;
     CUtensorMap tmA, tmB;
     int rc;
@@ -551,22 +565,20 @@ int run_conv(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &
         CUtensorMap tmU;
         rc = make_tmap_tiled(&tmU, kind_tm(pl.kind), io.w, pl.w_pitch, g.OC, 0, (uint64_t)pl.w_pitch * pl.es, 0, pl.slab_elems, UNIT_BN, pl.slab_bytes);
         if (rc != ONE_OK) return rc;
-        t_last_split = u.splits;
-        t_last_unit = 1;
+        note_form(UNIT_BN, u.splits, " unit");
         cudaError_t ce = launch_unit(pl.kind, tmA, tmU, p, u, stream);
         return ce == cudaSuccess ? ONE_OK : cuda_fail(ce, "unit launch");
     }
-    t_last_unit = 0;
     if (io.y_nchw) p.nchw_hw = g.OH * g.OW;
     if (!io.y_nchw && !pl.cta2 && pl.mh == 1 && pl.nw == 8 && split_eligible(pl.kind, p)) {
         int per = 0;
         const int splits = choose_split(ctx, M, g.OC, pl.bn, pl.num_kb, &per);
         if (splits > 1 && (rc = run_split(ctx, pl.kind, pl.bn, tmA, tmB, p, splits, per, stream)) != 1) {
-            t_last_split = splits;
+            note_form(pl.bn, splits, "");
             return rc;
         }
     }
-    t_last_split = 1;
+    note_form(pl.bn, 1, form_name(pl.cta2, pl.mh, pl.nw));
     CUtensorMap tmC, tmR, tmI;
     // Residual added by the tensor core (bit 3 of the epilogue mode): a 16-bit residual of the operands' own
     // format, no activation between the convolution and the Add, plain 256-wide tiles on full 128-byte slabs
@@ -641,6 +653,11 @@ int run_gemm(one_ctx *ctx, int kind, const void *A, int a_pitch, const void *B, 
              cudaStream_t stream, const GemmEpi *epi = nullptr)
 {
     if (M > 0x7fffffffLL) return fail(ONE_ERR_BAD_SHAPE, "GEMM: M too large");
+    const bool prepared = tmB_cached != nullptr;   // (a kept map is a prepared operator's)
+    if (plain_for_split(auto_tile, kind)) {
+        if (tile_cta2(bn)) tmB_cached = nullptr;   // its box is half a tile
+        bn = tile_bn(bn);
+    }
     const bool cta2 = tile_cta2(bn) && batch == 0;   // `bn` arrives as a tile code; a batched product stays single-CTA
     const int mh = tile_mh(bn), nw = batch == 0 ? tile_nw(bn) : 8;
     bn = tile_bn(bn);
@@ -660,20 +677,20 @@ int run_gemm(one_ctx *ctx, int kind, const void *A, int a_pitch, const void *B, 
     p.bias_mode = bias ? BIAS_F32 : BIAS_NONE; p.bias = bias;
     if (epi) { p.act = epi->act; p.lut = epi->lut; p.residual = epi->residual; }
     p.lut_smem = p.act == SILU && p.lut && !p.residual && (reinterpret_cast<uintptr_t>(p.lut) & 15) == 0;
-    p.consts = tmB_cached != nullptr;   // (a cached map is a prepared operator's)
+    p.consts = prepared;
     p.status = ctx->status_dev;
     UnitParams u;
     memset(&u, 0, sizeof(u));
     u.b_const = p.consts;
-    t_last_unit = (u.splits = choose_unit(auto_tile, M, N, batch, p.num_kb)) && unit_epilogue(kind, p, u) >= 0;
-    if (tmB_cached && !t_last_unit) tmB = *tmB_cached;
+    const bool unit = (u.splits = choose_unit(auto_tile, M, N, batch, p.num_kb)) && unit_epilogue(kind, p, u) >= 0;
+    if (tmB_cached && !unit) tmB = *tmB_cached;
     else {
         rc = make_tmap_tiled(&tmB, kind_tm(kind), B, K, N, batch, (uint64_t)b_pitch * es, (uint64_t)b_bstride * es,
-                             slab_elems, t_last_unit ? UNIT_BN : (cta2 ? bn / 2 : bn), slab_bytes);
+                             slab_elems, unit ? UNIT_BN : (cta2 ? bn / 2 : bn), slab_bytes);
         if (rc != ONE_OK) return rc;
     }
-    if (t_last_unit) {
-        t_last_split = u.splits;
+    if (unit) {
+        note_form(UNIT_BN, u.splits, " unit");
         cudaError_t ce = launch_unit(kind, tmA, tmB, p, u, stream);
         return ce == cudaSuccess ? ONE_OK : cuda_fail(ce, "unit launch");
     }
@@ -681,11 +698,11 @@ int run_gemm(one_ctx *ctx, int kind, const void *A, int a_pitch, const void *B, 
         int per = 0;
         const int splits = choose_split(ctx, M, N, bn, p.num_kb, &per);
         if (splits > 1 && (rc = run_split(ctx, kind, bn, tmA, tmB, p, splits, per, stream)) != 1) {
-            t_last_split = splits;
+            note_form(bn, splits, "");
             return rc;
         }
     }
-    t_last_split = 1;
+    note_form(bn, 1, form_name(cta2, mh, nw));
     CUtensorMap tmC, tmR;
     if ((rc = make_store_map(kind, &tmC, &tmR, &p.tma_store, out, out_mode, M, N, ldo, batch, out_bstride, p.residual, nullptr)) != ONE_OK) return rc;
     if (!vec_constants_ok(p)) p.tma_store = 0;
@@ -728,18 +745,26 @@ inline bool overlap(const void *a, size_t a_bytes, const void *b, size_t b_bytes
     return x < y + b_bytes && y < x + a_bytes;
 }
 
-// A convolution whose output is the reference layout, written by the epilogue itself -- or, when `out` shares memory with a
-// tensor that the launch reads (an earlier CTA's output would be another's bias or table), through an NHWC copy in the workspace.
-// Input and weights have been copied into the workspace by then.
+// A convolution whose output is the reference layout, written by the epilogue itself -- or by way of an NHWC copy in the
+// workspace, when
+//  * `out` shares memory with a tensor that the launch reads (an earlier CTA's output would be another's bias or table;
+//    input and weights have been copied into the workspace by then), or
+//  * the launch splits K over scratch planes, whose sum is written in rows.  A 3x3 512 -> 512 on 28 x 28 pixels is 56 tiles
+//    of 144 K blocks, a 7x7 512 -> 512 on 7 x 7 eight of 784: 8 CTAs in 315 us where 128 take 147.
 int run_conv_nchw(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &pl, ConvIO io, const CUtensorMap *tmB_cached,
                   float *out, cudaStream_t stream)
 {
     const long long M = (long long)g.N * g.OH * g.OW;
     const size_t out_bytes = (size_t)M * g.OC * 4;
     io.out_mode = OUT_F32;
-    if ((io.bias && overlap(out, out_bytes, io.bias, (size_t)g.OC * 4)) || (e.act == SILU && overlap(out, out_bytes, io.lut, 8192 * 4))) {
-        void *yh = ws_alloc(ctx, out_bytes);
-        if (!yh) return fail(ONE_ERR_NOMEM, "Conv: workspace too small for the NHWC output");
+    const bool shared = (io.bias && overlap(out, out_bytes, io.bias, (size_t)g.OC * 4)) || (e.act == SILU && overlap(out, out_bytes, io.lut, 8192 * 4));
+    const bool unit = choose_unit(pl.auto_tile, M, g.OC, 0, pl.num_kb) && !(e.act == SILU && (reinterpret_cast<uintptr_t>(io.lut) & 15));
+    int per;
+    const bool split = !unit && pl.kind != KIND_I8 && g.OC % 4 == 0 && (reinterpret_cast<uintptr_t>(io.bias) & 15) == 0 &&
+                       ((!pl.cta2 && pl.mh == 1 && pl.nw == 8) || plain_for_split(pl.auto_tile, pl.kind)) && choose_split(ctx, M, g.OC, pl.bn, pl.num_kb, &per) > 1;
+    void *yh = shared || split ? ws_alloc(ctx, out_bytes) : nullptr;
+    if (shared && !yh) return fail(ONE_ERR_NOMEM, "Conv: workspace too small for the NHWC output");
+    if (yh) {
         io.y = yh;
         int rc = run_conv(ctx, g, e, pl, io, tmB_cached, stream);
         if (rc != ONE_OK) return rc;
@@ -789,8 +814,7 @@ int run_raw(one_ctx *ctx, int kind, const float *A, const float *B, int b_kn, lo
     if (!u.a_ld) rc = make_tmap_tiled(&tmA, TM_F32, A, K, M, batch, (uint64_t)K * 4, (uint64_t)u.a_bstride * 4, p.slab_elems, 128, slab_bytes);
     if (rc == ONE_OK && !u.b_ld) rc = make_tmap_tiled(&tmB, TM_F32, B, K, N, batch, (uint64_t)K * 4, (uint64_t)u.b_bstride * 4, p.slab_elems, UNIT_BN, slab_bytes);
     if (rc != ONE_OK) return rc;
-    t_last_split = u.splits;
-    t_last_unit = 1;
+    note_form(UNIT_BN, u.splits, " unit");
     cudaError_t ce = launch_unit(kind, tmA, tmB, p, u, stream);
     return ce == cudaSuccess ? ONE_OK : cuda_fail(ce, "unit launch");
 }
@@ -1155,6 +1179,13 @@ extern "C" int one_cuda_packed_detail(one_packed *op, char *buf, size_t cap)
     return ONE_OK;
 }
 
+extern "C" int one_cuda_last_form(char *buf, size_t cap)
+{
+    if (!buf || !cap) return fail(ONE_ERR_BAD_ARG, "one_cuda_last_form: null argument");
+    snprintf(buf, cap, "tile=128x%d split=%d%s", t_last.bn, t_last.split, t_last.how);
+    return ONE_OK;
+}
+
 extern "C" int one_cuda_packed_work(one_packed *op, double *flops, double *bytes)
 {
     if (!op) return fail(ONE_ERR_BAD_ARG, "null operator");
@@ -1410,8 +1441,8 @@ extern "C" int one_cuda_eval_async(one_ctx *ctx, one_packed *op, BUFFER_INFO_S *
             if ((rc = run_conv(ctx, gl, op->e, op->pl, io, &op->tmB, st)) != ONE_OK) return rc;
         }
         snprintf(op->detail, sizeof(op->detail), "M=%lld N=%d K=%d %dx%d/%d C=%d@%dx%d %s tile=128x%d split=%d%s%s", M, g.OC, g.C * g.KH * g.KW, g.KH, g.KW,
-                 g.sh, g.C, g.H, g.W, kind_name(op->kind), op->pl.bn, t_last_split,
-                 op->paired ? " paired" : "", t_last_unit ? " unit" : op->pl.cta2 ? " 2cta" : (op->pl.mh == 2 ? " 2half" : (op->pl.nw == 12 ? " 12w" : "")));
+                 g.sh, g.C, g.H, g.W, kind_name(op->kind), t_last.bn, t_last.split,
+                 op->paired ? " paired" : "", t_last.how);
         op->flops = 2.0 * (double)M * g.OC * g.C * g.KH * g.KW;   // host/ops/conv.h:159-176
         const double aes = (op->flags & ONE_IN_S8) ? 1.0 : (op->e.int8 ? 4.0 : (nhwc && bf16 ? 2.0 : 4.0));
         const double yes = outputs[0].addr ? ((nhwc && ((bf16 && !(op->flags & ONE_OUT_F32)) || (op->flags & ONE_OUT_BF16))) ? 2.0 : 4.0) : 0.0;
@@ -1454,8 +1485,7 @@ extern "C" int one_cuda_eval_async(one_ctx *ctx, one_packed *op, BUFFER_INFO_S *
                       reinterpret_cast<void *>(outputs[0].addr), op->N, 0, out_mode, reinterpret_cast<const float *>(op->bias),
                       &op->tmB, op->bn, op->auto_tile, st, &epi);
     if (rc != ONE_OK) return rc;
-    snprintf(op->detail, sizeof(op->detail), "M=%lld N=%d K=%d %s tile=128x%d split=%d%s", rows, op->N, op->K, kind_name(op->kind), tile_bn(op->bn),
-             t_last_split, t_last_unit ? " unit" : tile_cta2(op->bn) ? " 2cta" : (tile_mh(op->bn) == 2 ? " 2half" : (tile_nw(op->bn) == 12 ? " 12w" : "")));
+    snprintf(op->detail, sizeof(op->detail), "M=%lld N=%d K=%d %s tile=128x%d split=%d%s", rows, op->N, op->K, kind_name(op->kind), t_last.bn, t_last.split, t_last.how);
     op->flops = 2.0 * (double)rows * op->N * op->K;
     op->bytes = (double)rows * op->K * (a_native ? es : 4) + (double)op->N * op->K * es +
                 (double)rows * op->N * (out_is_16(out_mode) ? 2 : 4) * (epi.residual ? 2 : 1);

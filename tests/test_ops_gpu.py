@@ -273,8 +273,14 @@ def test_conv_split_k_vs_oracle_and_unsplit(ops, oracle_mod, case, splits):
     try:
         capi.check(L.one_cuda_set_split_k(1))
         y1 = _np(ops.conv(x, w, b, (s, s), (pad,) * 4, act, lut=lut))
+        assert capi.last_form().endswith("split=1")
         capi.check(L.one_cuda_set_split_k(splits))
         ys = _np(ops.conv(x, w, b, (s, s), (pad,) * 4, act, lut=lut))
+        form = capi.last_form()
+        if splits:      # that many ranges, or the whole number of K blocks each that comes closest
+            assert "unit" not in form and 2 <= int(form.split("split=")[1]) <= splits, form
+        else:
+            assert "unit" in form, form
         ys2 = _np(ops.conv(x, w, b, (s, s), (pad,) * 4, act, lut=lut))
     finally:
         L.one_cuda_set_split_k(0)
@@ -297,6 +303,9 @@ def test_gemm_split_k_vs_oracle(ops, oracle_mod, shape, splits):
     try:
         capi.check(L.one_cuda_set_split_k(splits))
         y = _np(ops.gemm(a, w, b))
+        blocks = -(-K // 32)      # K blocks; a range holds a whole number of them
+        ranges = -(-blocks // -(-blocks // min(splits, blocks))) if splits else 0
+        assert "unit" in capi.last_form() if splits == 0 else capi.last_form().endswith(f"split={ranges}")
     finally:
         L.one_cuda_set_split_k(0)
     assert_close(y, oracle_mod.gemm(a, w, b), f"gemm {shape} split {splits}")
@@ -503,11 +512,20 @@ def test_one_wave_gemm_and_matmul_vs_oracle_and_persistent(ops, oracle_mod, shap
     b3 = (rng.standard_normal((2, K, N)) * 0.05).astype(np.float32)
     L = capi.lib()
     capi.check(L.one_cuda_set_eval_precision(capi.PRECISIONS[prec]))
+    def unit(rows, batch):     # all of the launch's 128 x 64 tiles are resident at once
+        return -(-rows // 128) * -(-N // 64) * batch <= 296
+
+    def call(fn, rows, batch, *args):
+        y = _np(fn(*args))
+        assert ("unit" in capi.last_form()) == unit(rows, batch), capi.last_form()
+        return y
+
     try:
-        got = [_np(ops.gemm(a, w, b)), _np(ops.matmul(a3, b3)), _np(ops.matmul(a3, b3[0]))]
+        got = [call(ops.gemm, M, 1, a, w, b), call(ops.matmul, M, 2, a3, b3), call(ops.matmul, 2 * M, 1, a3, b3[0])]
         again = [_np(ops.gemm(a, w, b)), _np(ops.matmul(a3, b3)), _np(ops.matmul(a3, b3[0]))]
         capi.check(L.one_cuda_set_split_k(1))
         plain = [_np(ops.gemm(a, w, b)), _np(ops.matmul(a3, b3)), _np(ops.matmul(a3, b3[0]))]
+        assert "unit" not in capi.last_form()
     finally:
         L.one_cuda_set_split_k(0)
         L.one_cuda_set_eval_precision(capi.PREC_TF32)
@@ -537,10 +555,14 @@ def test_one_wave_conv_vs_oracle_and_persistent(ops, oracle_mod, case):
     lut = oracle_mod.silu_lut() if act == abi.SILU else None
     w8, b32, aux = oracle_mod.quant_weight_bias(w, b)
     L = capi.lib()
-    y, y8 = _np(ops.conv(x, w, b, (s, s), (p,) * 4, act, lut=lut)), _np(ops.conv(x, w8, b32, (s, s), (p,) * 4, act, int8=(0.01, aux), lut=lut))
+    y = _np(ops.conv(x, w, b, (s, s), (p,) * 4, act, lut=lut))
+    assert "unit" in capi.last_form()
+    y8 = _np(ops.conv(x, w8, b32, (s, s), (p,) * 4, act, int8=(0.01, aux), lut=lut))
+    assert "unit" in capi.last_form()
     try:
         capi.check(L.one_cuda_set_split_k(1))
         z, z8 = _np(ops.conv(x, w, b, (s, s), (p,) * 4, act, lut=lut)), _np(ops.conv(x, w8, b32, (s, s), (p,) * 4, act, int8=(0.01, aux), lut=lut))
+        assert "unit" not in capi.last_form()
     finally:
         L.one_cuda_set_split_k(0)
     ref = oracle_mod.conv_f32(x, w, b, (s, s), (p,) * 4, act)
@@ -550,11 +572,11 @@ def test_one_wave_conv_vs_oracle_and_persistent(ops, oracle_mod, case):
     assert np.array_equal(y8, ref8) and np.array_equal(z8, ref8)
 
 
-# precision, N, C, H, W, OC, k, stride, the plain tile: one launch of each form that the library chooses by itself, just
+# precision, N, C, H, W, OC, k, stride, the plain tile, the chosen form: one launch of each form that the library chooses by itself, just
 # above the size from which it does
 CHOSEN_FORMS = [
-    ("int8", 1, 3, 560, 560, 32, 3, 2, 64), ("int8", 1, 128, 200, 200, 128, 1, 1, 128), ("f16", 1, 128, 150, 151, 128, 3, 1, 128),
-    ("f16", 1, 512, 390, 390, 128, 1, 1, 128), ("f16", 1, 512, 195, 195, 256, 1, 1, 256), ("tf32", 1, 3, 560, 562, 48, 7, 2, 64),
+    ("int8", 1, 3, 560, 560, 32, 3, 2, 64, "2half"), ("int8", 1, 128, 200, 200, 128, 1, 1, 128, "12w"), ("f16", 1, 128, 150, 151, 128, 3, 1, 128, "2half"),
+    ("f16", 1, 512, 390, 390, 128, 1, 1, 128, "2cta"), ("f16", 1, 512, 195, 195, 256, 1, 1, 256, "2cta"), ("tf32", 1, 3, 560, 562, 48, 7, 2, 64, "2half"),
 ]
 
 
@@ -562,7 +584,7 @@ CHOSEN_FORMS = [
 def test_chosen_tile_form_equals_plain_tiles(ops, oracle_mod, case):
     """Halves, pairs and twelve epilogue warps add the same products in the same order as single CTAs: the same bits."""
     import torch
-    prec, N, C, H, W, OC, k, s, tile = case
+    prec, N, C, H, W, OC, k, s, tile, form = case
     gen = torch.Generator(device="cuda").manual_seed(C + OC + H)
     x = torch.rand((N, C, H, W), generator=gen, device="cuda") * 2 - 1
     w = (torch.randn((OC, C, k, k), generator=gen, device="cuda") * 0.05).cpu().numpy()
@@ -578,9 +600,18 @@ def test_chosen_tile_form_equals_plain_tiles(ops, oracle_mod, case):
     capi.check(L.one_cuda_set_eval_precision(capi.PRECISIONS["tf32" if prec == "int8" else prec]))
     try:
         y = run()
+        assert capi.last_form().endswith(" " + form), capi.last_form()
         capi.check(L.one_cuda_set_tile_n(tile))
         z = run()
+        assert capi.last_form() == f"tile=128x{tile} split=1"
+        if prec != "int8":      # a forced number of K ranges takes plain tiles, whatever would have been chosen
+            L.one_cuda_set_tile_n(0)
+            capi.check(L.one_cuda_set_split_k(2))
+            v = run()
+            assert capi.last_form() in (f"tile=128x{tile} split=2", f"tile=128x{tile} split=1")    # (1: the planes do not fit)
+            assert (v - z).norm() <= 1e-5 * z.norm()
     finally:
+        L.one_cuda_set_split_k(0)
         L.one_cuda_set_tile_n(0)
         L.one_cuda_set_eval_precision(capi.PREC_TF32)
     assert torch.equal(y, z) and bool(y.any())
@@ -682,3 +713,55 @@ def test_output_that_shares_memory_with_an_input(ops):
                                       inside.data_ptr() if name == "table" else table.data_ptr())
             capi.check(capi.shim_eval("Conv")(args.params, args.inputs, args.outputs))
             assert torch.equal(pool[:want.numel()].view_as(want), want), (OC, name)
+
+
+# C, H, W, OC, k, the K ranges the library takes: few tiles with a K range too long for the one-wave kernel
+LONG_K = [(512, 7, 7, 512, 7, 16), (512, 28, 28, 512, 3, 2), (256, 9, 11, 36, 9, 16)]
+
+
+@pytest.mark.parametrize("case", LONG_K, ids=[f"{c[0]}to{c[3]}k{c[4]}@{c[1]}x{c[2]}" for c in LONG_K])
+def test_long_k_ranges_into_the_reference_layout_are_split(ops, oracle_mod, case):
+    """A reference-layout output does not keep the library from splitting K over scratch planes."""
+    C, H, W, OC, k, want = case
+    rng = np.random.default_rng(C + OC)
+    x = rng.uniform(-1, 1, (1, C, H, W)).astype(np.float32)
+    w = (rng.standard_normal((OC, C, k, k)) * 0.02).astype(np.float32)
+    b = rng.standard_normal(OC).astype(np.float32)
+    y = _np(ops.conv(x, w, b, (1, 1), (k // 2,) * 4, abi.RELU))
+    assert capi.last_form().endswith(f"split={want}"), capi.last_form()
+    L = capi.lib()
+    try:
+        capi.check(L.one_cuda_set_split_k(1))
+        z = _np(ops.conv(x, w, b, (1, 1), (k // 2,) * 4, abi.RELU))
+    finally:
+        L.one_cuda_set_split_k(0)
+    assert_close(y, oracle_mod.conv_f32(x, w, b, (1, 1), (k // 2,) * 4, abi.RELU), str(case))
+    # each of the K / 8 accumulation steps drops less than a unit in the last place of a running sum
+    assert np.linalg.norm(y - z) <= C * k * k / 8 * 2.0 ** -23 * np.linalg.norm(z)
+
+
+def test_forced_split_of_a_prepared_product_that_would_run_as_pairs():
+    """The split count of a prepared operator is honoured where the library's own choice is a pair of CTAs."""
+    import torch
+    M, K, N = 38000, 256, 192
+    rng = np.random.default_rng(9)
+    w, b = (rng.standard_normal((N, K)) * 0.1).astype(np.float32), rng.standard_normal(N).astype(np.float32)
+    a = torch.randn((M, K), device="cuda")
+    y = torch.empty((M, N), device="cuda")
+    ctx = capi.Context(0, 1 << 28)
+    op = capi.Packed(ctx, "Gemm", abi.gemm_eval_args((M, K), (N, K), (M, N), 0, w.ctypes.data, b.ctypes.data, 0), capi.LAYOUT_NHWC)
+    args = abi.gemm_eval_args((M, K), (N, K), (M, N), a.data_ptr(), 0, 0, y.data_ptr())
+    torch.cuda.synchronize()
+    try:
+        out = []
+        for splits, form in ((0, "split=1 2cta"), (2, "split=2"), (0, "split=1 2cta")):
+            capi.check(capi.lib().one_cuda_packed_set_split(op.handle, splits))
+            op.eval_async(args)
+            assert capi.last_form().endswith(form), capi.last_form()
+            ctx.status()
+            out.append(y.clone())
+        assert torch.equal(out[0], out[2]) and (out[1] - out[0]).norm() <= 1e-5 * out[0].norm()
+        assert (out[0] - (a.double() @ torch.from_numpy(w).cuda().double().t() + torch.from_numpy(b).cuda()).float()).norm() <= 2e-3 * out[0].norm()
+    finally:
+        op.close()
+        ctx.close()
