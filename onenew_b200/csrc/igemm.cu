@@ -315,8 +315,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     // accesses are ordered after it.  The next kernel may start its own prologue right away; it cannot
     // touch data before its own wait, which in turn covers this whole grid.
     // (The release of the next launch comes first: its blocks then do their own set-up while this one waits.)
-    // The epilogue's read-only loads (bias, coefficients, a table in global memory) stand behind the branch on the warp's
-    // role and the loop over tiles: a load that may not be executed is not moved up here, so their pointers need no laundering.
+    // The wait does not order read-only loads either (see launch.cuh), and the epilogue reads bias and coefficients with such.
+    // They and the table are a prepared operator's copies, or a drop-in call's tensors: see FirstLaunchPlain for those.
     if (p.pdl) {
         pdl_launch_dependents();
         pdl_wait();
@@ -1108,8 +1108,8 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const SplitKReducePa
         pdl_launch_dependents();
         pdl_wait();
     }
-    const float *partial = p.partial, *bias = p.bias, *lut = p.lut;
-    launder(partial); launder(bias); launder(lut);   // no load of theirs above the wait
+    const float *partial = p.partial;
+    launder(partial);   // (no load of the planes above the wait; bias and table by plain loads)
     const bool out16 = out_is_16(p.out_mode), f16 = p.out_mode == OUT_F16;
     float vmax = 0.f;
     const long long quads_per_row = p.N >> 2;
@@ -1125,16 +1125,16 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const SplitKReducePa
             acc.z = __fadd_rn(acc.z, t.z); acc.w = __fadd_rn(acc.w, t.w);
         }
         float v[4] = {acc.x, acc.y, acc.z, acc.w};
-        if (bias) {
+        if (p.bias) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = __fadd_rn(v[e], __ldg(bias + n + e));
+            for (int e = 0; e < 4; ++e) v[e] = __fadd_rn(v[e], p.bias[n + e]);
         }
         if (p.act == 1) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = v[e] > 0.f ? v[e] : 0.f;
         } else if (p.act != 0) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = apply_act(v[e], p.act, p.act_p0, p.act_p1, lut);
+            for (int e = 0; e < 4; ++e) v[e] = apply_act(v[e], p.act, p.act_p0, p.act_p1, p.lut);
         }
         const long long off = m * p.ldo + n;
         if (p.residual) {
@@ -1243,10 +1243,7 @@ static cudaError_t launch_one(const CUtensorMap &tmA, const CUtensorMap &tmB, co
     const long long sms = sm_count_of(dev);
     const long long slots = PAIR ? sms / 2 : sms;
     const unsigned grid = (unsigned)(tiles < slots ? tiles : slots) * (PAIR ? 2u : 1u);
-    // A table that is the caller's may have been written by the launch before this one, and the kernel stages it before its
-    // wait: such a call is launched plainly.  (Staging it after the wait instead costs every other launch: the second copy
-    // of the loop and its barrier slowed the int8 backbone of 64 images from 1614 to 1649 us.)
-    p.pdl = get_pdl() && (p.consts || !p.lut_smem);
+    p.pdl = get_pdl();
     p.epi_mode = g_epi_mode.load(std::memory_order_relaxed);
     cudaError_t e = launch_ex(igemm_kernel<KIND, BN, PAIR, MH, NEW>, dim3(grid), dim3(num_threads_for(NEW)), smem, stream, p.pdl != 0, PAIR ? 2 : 1, tmA, tmB, tmC, tmR, tmI, p);
     count_launch();

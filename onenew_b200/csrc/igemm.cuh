@@ -40,9 +40,6 @@ struct IgemmParams {
     const float *lut;     // SiLU / Gelu table (8192 entries)
     int q_table;          // int8: no NaN can come out of the de-quantisation (finite coefficients, a scale below 2^90)
     int lut_smem;         // stage the table in shared memory (only without a residual; 16-byte aligned table)
-    int consts;           // bias, coefficients and table are a prepared operator's own copies: no kernel of the stream writes
-                          // them, so they may be read before the wait for the previous launch.  A drop-in call reads the
-                          // caller's tensors, which that launch may still be writing.
     const void *residual; // optional [M][ldo], same element type as out; added before res_relu
     int res_relu;         // relu after the residual add
     int nchw_hw;          // > 0: out is fp32 [M / hw][N][hw], the reference layout of a convolution's output (no residual,

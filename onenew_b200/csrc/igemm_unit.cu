@@ -154,10 +154,8 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         tmem_alloc(smem_u32(tmem_slot), BN);
         tmem_relinquish();
     }
-    auto stage_table = [&](const float4 *g4) {
-        for (int i = threadIdx.x; i < 2048; i += THREADS) reinterpret_cast<float4 *>(slut)[i] = __ldg(g4 + i);
-    };
-    if (has_lut && u.b_const) stage_table(reinterpret_cast<const float4 *>(p.lut));
+    if (has_lut)   // staged before the wait: a prepared operator's, or a drop-in call's (see FirstLaunchPlain)
+        for (int i = threadIdx.x; i < 2048; i += THREADS) reinterpret_cast<float4 *>(slut)[i] = __ldg(reinterpret_cast<const float4 *>(p.lut) + i);
     tc_fence_before_sync();
     __syncthreads();
     if constexpr (S > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // (waited for before the first write to a peer)
@@ -176,17 +174,17 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const int col = n0 + c0 + chunk * 4, nvalid = p.N - col;        // this lane's four columns in a row-major output
     const bool f16 = p.out_mode == OUT_F16;
     alignas(16) float cst_[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const float *gbias = reinterpret_cast<const float *>(p.bias), *gcoeff = p.coeff;
-    auto load_constants = [&]() {
-        if (ROWS && nvalid > 0) {
+    // (The caller's tensors may have been written by an earlier kernel of the stream.  Plain loads here and below: a read-only
+    // one, __ldg, is not ordered by the wait -- one behind a conditional wait was seen to run ahead of it.)
+    const float *bias = reinterpret_cast<const float *>(p.bias);
+    if (!u.b_const && p.pdl) pdl_wait();
+    if (ROWS && nvalid > 0) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (gbias) cst_[e] = __ldg(gbias + col + e);
-                if (KIND == KIND_I8) cst_[4 + e] = __ldg(gcoeff + col + e);
-            }
+        for (int e = 0; e < 4; ++e) {
+            if (bias) cst_[e] = bias[col + e];
+            if (KIND == KIND_I8) cst_[4 + e] = p.coeff[col + e];
         }
-    };
-    if (u.b_const) load_constants();
+    }
 
     const bool tma_a = !RAW || u.a_ld == 0, tma_b = !RAW || u.b_ld == 0;
     const uint32_t tx = (tma_a ? a_slab : 0u) + (tma_b ? b_slab : 0u);
@@ -262,17 +260,6 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     } else {
         if (p.pdl) pdl_wait();
     }
-    // The caller's tensors, which an earlier kernel of the stream may have written: read through laundered pointers, so that
-    // no read-only load of theirs can be moved above the wait (or merged with one that stands there).
-    launder(gbias); launder(gcoeff);
-    if (!u.b_const) {
-        load_constants();
-        if (has_lut) {
-            const float4 *g4 = reinterpret_cast<const float4 *>(p.lut);
-            launder(g4);
-            stage_table(g4);
-        }
-    }
     if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         const uint32_t idesc = make_idesc<KIND>(A_ROWS, BN) & ((KIND == KIND_BF16 && p.ab_f16) ? ~((7u << 7) | (7u << 10)) : ~0u);
@@ -311,8 +298,6 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             // 16-byte pieces of the K-major tiles: piece c of row r lies at c ^ (r & 7) within a 128-byte row (narrower
             // rows: the corresponding swizzle), so an in-place pass needs no addresses but the linear ones.
             const int t = threadIdx.x - 64;
-            const float *ga = u.a, *gb = u.b;
-            launder(ga); launder(gb);
             auto rnd4 = [](uint4 v) {
                 return make_uint4(__float_as_uint(round_to_tf32(__uint_as_float(v.x))), __float_as_uint(round_to_tf32(__uint_as_float(v.y))),
                                   __float_as_uint(round_to_tf32(__uint_as_float(v.z))), __float_as_uint(round_to_tf32(__uint_as_float(v.w))));
@@ -324,7 +309,7 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const bool in = row < rows && k + e < u.K;
-                    v[e] = in ? __ldg(mode == 2 ? base + (long long)(k + e) * pitch + row : base + (long long)row * pitch + k + e) : 0.f;
+                    v[e] = in ? *(mode == 2 ? base + (long long)(k + e) * pitch + row : base + (long long)row * pitch + k + e) : 0.f;
                 }
                 return make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
             };
@@ -338,7 +323,7 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 c = u.b_ld == 2 ? j / BN : j & (cpr - 1);
             };
             auto fetch_b = [&](int i) {
-                const float *base = gb + (long long)bz * u.b_bstride;
+                const float *base = u.b + (long long)bz * u.b_bstride;
 #pragma unroll
                 for (int q = 0; q < BPIECES; ++q) {
                     int r, c;
@@ -353,7 +338,7 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 const int k0 = (kb0 + i) * p.slab_elems;
                 if ((u.a_ld || u.b_ld) && i >= stages && !mbar_wait(empty0 + 8 * s, phase ^ 1, abort_flag)) ok = false;
                 if (ok && u.a_ld) {
-                    const float *base = ga + (long long)bz * u.a_bstride;
+                    const float *base = u.a + (long long)bz * u.a_bstride;
 #pragma unroll 3
                     for (int j = t; j < A_ROWS * cpr; j += 192) {
                         const int r = j >> cshift, c = j & (cpr - 1);
@@ -417,7 +402,6 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
     }
     bool got = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0, abort_flag));
-    if (has_lut && !u.b_const) __syncthreads();   // every warp's part of the table is in place
     // Block w of the tile passes through shared memory (the ring is free: every MMA of the tile has completed) as 32 rows
     // of 128 bytes, 16-byte piece c of row x at c ^ (x & 7).  A cluster deals the rows out in S slices, CTA z finishes
     // slice z: each warp sends every slice of its partial block to its owner, [source CTA][block][row of the slice].
@@ -542,7 +526,7 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 #pragma unroll
                 for (int z = 1; z < S; ++z) raw[0] = add_partial<KIND>(raw[0], *reinterpret_cast<const uint32_t *>(src + z * (NBLK * PER * 128)));
                 if (m >= p.M || n >= p.N) continue;
-                const float b[1] = {gbias ? __ldg(gbias + n) : 0.f}, k[1] = {KIND == KIND_I8 ? __ldg(gcoeff + n) : 0.f};
+                const float b[1] = {bias ? bias[n] : 0.f}, k[1] = {KIND == KIND_I8 ? p.coeff[n] : 0.f};
                 float t[1];
                 finish<KIND, 1>(t, raw, b, k, p, slut);
                 long long off;

@@ -8,8 +8,8 @@ namespace one {
 // tma_store, res_mma, nchw_hw and lut_smem are not read).
 struct UnitParams {
     int splits;           // CTAs of a cluster that share a tile along K: 1, 2, 4 or 8
-    int b_const;          // B holds a prepared operator's weights, and its bias, coefficients and table are the operator's own
-                          // copies: no earlier kernel of the stream writes them, so their loads start before the wait
+    int b_const;          // B holds a prepared operator's weights and bias its own copy: no earlier kernel of the stream writes
+                          // them, so their loads start before the wait
     int nchw_hw;          // > 0: out is fp32 [M / hw][N][hw] (the reference layout of a convolution's output)
     // fp32 operands read as the caller left them (tf32 launches with `raw`): rounded to tf32 on their way through
     // shared memory.  0: by TMA, K-major; 1: by plain loads, K-major rows of `pitch` floats; 2: by plain loads,

@@ -18,6 +18,20 @@ namespace one {
 
 int get_pdl();
 
+// A call on the caller's own tensors (the drop-in operators): its first launch has no such attribute.  That launch therefore
+// starts when everything before it on the stream has completed, and so does all that follows within the call: its kernels may
+// read the caller's tensors (the activation table, the bias) ahead of their own wait, which only has to order them behind each
+// other.  Without it a contraction could stage a table that a kernel before the call was still writing, since each of the launches
+// between the two releases its successor at once.  The stream is usually idle at that point, and the launch costs nothing more;
+// ordering the reads inside the contraction kernels did (int8 backbone of 64 images 1614 -> 1649 us), and so did launching the
+// contraction plainly (3 - 4 us of every drop-in Conv).
+struct FirstLaunchPlain {
+    static inline thread_local bool pending = false;
+    FirstLaunchPlain() { pending = true; }
+    ~FirstLaunchPlain() { pending = false; }
+    static bool take() { const bool p = pending; pending = false; return p; }
+};
+
 // Launch with the programmatic-stream-serialisation attribute when `pdl`, and as clusters of `cluster` CTAs when
 // that is above 1.
 template <typename... KArgs, typename... Args>
@@ -31,7 +45,7 @@ inline cudaError_t launch_ex(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int n = 0;
-    if (pdl) {
+    if (!FirstLaunchPlain::take() && pdl) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
         ++n;
@@ -59,7 +73,8 @@ inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
 template <typename P> __device__ __forceinline__ void launder(P &p) { asm volatile("" : "+l"(p)); }
 // Start of a kernel launched by launch_k: the next launch may be placed, this one waits until the previous kernel
 // has completed and its writes are visible.  The pointers the kernel reads through are passed here so that the
-// compiler cannot move a load through a `const __restrict__` pointer above the wait.
+// compiler cannot turn loads through a `const __restrict__` pointer into read-only ones (ld.global.nc), or move them above the
+// wait: the wait does not order read-only loads.  So no __ldg of what an earlier kernel may have written either.
 template <typename... P> __device__ __forceinline__ void pdl_entry(P &...ptrs)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

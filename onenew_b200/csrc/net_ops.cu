@@ -220,7 +220,7 @@ __global__ void k_maxpool3x3s2_nhwc_p16(const uint4 *__restrict__ x, uint4 *__re
 #pragma unroll
             for (int b = 0; b < 5; ++b) {
                 const int iw = ow0 * 2 + b - pad;
-                v[a][b] = (ih >= 0 && ih < H && iw >= 0 && iw < W) ? __ldg(x + (((size_t)n * H + ih) * W + iw) * cv + c) : ninf;
+                v[a][b] = (ih >= 0 && ih < H && iw >= 0 && iw < W) ? x[(((size_t)n * H + ih) * W + iw) * cv + c] : ninf;
             }
         }
         uint4 col[5];   // maxima down the three rows, then across three columns for each of the two outputs

@@ -29,6 +29,7 @@
 #include "glue.cuh"
 #include "igemm.cuh"
 #include "igemm_unit.cuh"
+#include "launch.cuh"
 #include "sm100_prims.cuh"
 
 using namespace one;
@@ -556,7 +557,6 @@ int run_conv(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &
     p.lut_smem = p.act == SILU && p.lut && !p.residual && (reinterpret_cast<uintptr_t>(p.lut) & 15) == 0;
     p.out_q = io.out_q; p.q_inv_scale = io.q_inv_scale;
     p.q_table = pl.kind == KIND_I8 && io.coeff_finite && fabsf(e.in_scale) < 0x1p90f;
-    p.consts = io.w_const;
     p.status = ctx->status_dev;
     UnitParams u;
     memset(&u, 0, sizeof(u));
@@ -677,11 +677,10 @@ int run_gemm(one_ctx *ctx, int kind, const void *A, int a_pitch, const void *B, 
     p.bias_mode = bias ? BIAS_F32 : BIAS_NONE; p.bias = bias;
     if (epi) { p.act = epi->act; p.lut = epi->lut; p.residual = epi->residual; }
     p.lut_smem = p.act == SILU && p.lut && !p.residual && (reinterpret_cast<uintptr_t>(p.lut) & 15) == 0;
-    p.consts = prepared;
     p.status = ctx->status_dev;
     UnitParams u;
     memset(&u, 0, sizeof(u));
-    u.b_const = p.consts;
+    u.b_const = prepared;
     const bool unit = (u.splits = choose_unit(auto_tile, M, N, batch, p.num_kb)) && unit_epilogue(kind, p, u) >= 0;
     if (tmB_cached && !unit) tmB = *tmB_cached;
     else {
@@ -940,6 +939,7 @@ extern "C" int one_cuda_set_launch_overlap(int on)
 
 extern "C" int one_cuda_conv_eval(BUFFER_INFO_S *params, BUFFER_INFO_S *inputs, BUFFER_INFO_S *outputs)
 {
+    FirstLaunchPlain plain;
     ConvGeom g; ConvEpi e; const CONV_CONFIG_S *cfg;
     int rc = parse_conv(params, &g, &e, &cfg);
     if (rc != ONE_OK) return rc;
@@ -1006,6 +1006,7 @@ extern "C" int one_cuda_conv_eval(BUFFER_INFO_S *params, BUFFER_INFO_S *inputs, 
 
 extern "C" int one_cuda_gemm_eval(BUFFER_INFO_S *params, BUFFER_INFO_S *inputs, BUFFER_INFO_S *outputs)
 {
+    FirstLaunchPlain plain;
     if (!params || !params[1].addr || !params[4].addr) return fail(ONE_ERR_BAD_ARG, "Gemm: params[1] / params[4] descriptors are null");
     if (!inputs || !outputs || !inputs[0].addr || !inputs[1].addr || !inputs[2].addr || !outputs[0].addr)
         return fail(ONE_ERR_BAD_ARG, "Gemm: null tensor pointer");
@@ -1088,6 +1089,7 @@ static int matmul_enqueue(one_ctx *ctx, int kind, BUFFER_INFO_S *params, BUFFER_
 
 extern "C" int one_cuda_matmul_eval(BUFFER_INFO_S *params, BUFFER_INFO_S *inputs, BUFFER_INFO_S *outputs)
 {
+    FirstLaunchPlain plain;
     MatmulShape s;   // descriptors are checked before anything touches the device
     int rc = parse_matmul(params, &s);
     if (rc != ONE_OK) return rc;
@@ -1529,6 +1531,7 @@ std::mutex g_static_mu;
 extern "C" int one_cuda_conv_eval_static(BUFFER_INFO_S *params, BUFFER_INFO_S *inputs, BUFFER_INFO_S *outputs,
                                          void *stream)
 {
+    FirstLaunchPlain plain;
     ConvGeom g; ConvEpi e; const CONV_CONFIG_S *cfg;
     int rc = parse_conv(params, &g, &e, &cfg);
     if (rc != ONE_OK) return rc;
