@@ -749,7 +749,13 @@ inline bool overlap(const void *a, size_t a_bytes, const void *b, size_t b_bytes
 //  * `out` shares memory with a tensor that the launch reads (an earlier CTA's output would be another's bias or table;
 //    input and weights have been copied into the workspace by then), or
 //  * the launch splits K over scratch planes, whose sum is written in rows.  A 3x3 512 -> 512 on 28 x 28 pixels is 56 tiles
-//    of 144 K blocks, a 7x7 512 -> 512 on 7 x 7 eight of 784: 8 CTAs in 315 us where 128 take 147.
+//    of 144 K blocks, a 7x7 512 -> 512 on 7 x 7 eight of 784: 8 CTAs in 315 us where 128 take 147; or
+//  * the persistent kernel can write rows of whole 32-column patches by TMA: 4-byte stores of a lane each take longer than that
+//    and a second pass over the output.  Direct / by way of the copy, us a call over 1x1 and 3x3 filters of 16 - 256 channels in
+//    tf32, fp16 and int8: 32 columns 43 / 34 to 150 / 139, 64 columns 58 / 37 to 136 / 93, 256 columns 88 / 47 to 273 / 148, 512
+//    columns 204 / 79.  Of the ragged widths only those of more than 128 columns gain, and only from a large output on: 132 and
+//    343 columns of 20 - 120 MB 1.00 - 1.17 times, 355 columns of 227 MB 654 / 586, but 159 columns of 2.6 MB 154 / 159; 33 and
+//    40 columns 44 / 54 to 67 / 93, 100 and 101 columns 0.84 - 1.14 times.
 int run_conv_nchw(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &pl, ConvIO io, const CUtensorMap *tmB_cached,
                   float *out, cudaStream_t stream)
 {
@@ -761,7 +767,8 @@ int run_conv_nchw(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvP
     int per;
     const bool split = !unit && pl.kind != KIND_I8 && g.OC % 4 == 0 && (reinterpret_cast<uintptr_t>(io.bias) & 15) == 0 &&
                        ((!pl.cta2 && pl.mh == 1 && pl.nw == 8) || plain_for_split(pl.auto_tile, pl.kind)) && choose_split(ctx, M, g.OC, pl.bn, pl.num_kb, &per) > 1;
-    void *yh = shared || split ? ws_alloc(ctx, out_bytes) : nullptr;
+    const bool rows = !unit && ((g.OC % 32 == 0 && (reinterpret_cast<uintptr_t>(io.bias) & 15) == 0) || (g.OC > 128 && out_bytes >= (size_t(16) << 20)));
+    void *yh = shared || split || rows ? ws_alloc(ctx, out_bytes) : nullptr;
     if (shared && !yh) return fail(ONE_ERR_NOMEM, "Conv: workspace too small for the NHWC output");
     if (yh) {
         io.y = yh;

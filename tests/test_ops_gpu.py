@@ -765,3 +765,17 @@ def test_forced_split_of_a_prepared_product_that_would_run_as_pairs():
     finally:
         op.close()
         ctx.close()
+
+
+@pytest.mark.parametrize("OC", [32, 40, 96, 101, 132])
+def test_many_tiles_into_the_reference_layout(ops, oracle_mod, OC):
+    """Epilogue stores straight into NCHW, and by way of rows: widths on both sides of the line, a ragged last row tile."""
+    rng = np.random.default_rng(OC)
+    x = rng.uniform(-1, 1, (3, 16, 114, 113)).astype(np.float32)
+    w, b = (rng.standard_normal((OC, 16, 1, 1)) * 0.2).astype(np.float32), rng.standard_normal(OC).astype(np.float32)
+    w8, b32, aux = oracle_mod.quant_weight_bias(w, b)
+    y = _np(ops.conv(x, w, b, act=abi.LEAKYRELU))
+    assert ("unit" in capi.last_form()) == (-(-3 * 114 * 113 // 128) * -(-OC // 64) <= 296)
+    assert_close(y, oracle_mod.conv_f32(x, w, b, (1, 1), (0,) * 4, abi.LEAKYRELU), str(OC))
+    y8 = _np(ops.conv(x, w8, b32, act=abi.RELU, int8=(0.01, aux)))
+    assert np.array_equal(y8, oracle_mod.conv_s8(x, w8, b32, aux, 0.01, (1, 1), 0, abi.RELU)[0])
