@@ -204,7 +204,9 @@ int run_split(one_ctx *ctx, int kind, int bn, const CUtensorMap &tmA, const CUte
 // a long K range wants its 256-wide tiles, which bring half the operand bytes per product.  ResNet-50, us (limit of tiles /
 // of K blocks a CTA): fp16 32 images 1217 (148 / 64), 1195 (296 / 24), 1141 (296 / 64); TF32 61 images of 192 x 192: 2048,
 // 2037, 2021; without the unit kernel 1230 and 2022.  Few tiles are cut along K until the SMs are covered; a CTA keeps at
-// least two K blocks, since below that the exchange costs more than the blocks it saves.
+// least two K blocks, since below that the exchange costs more than the blocks it saves.  So few tiles that the persistent
+// kernel cuts them into 16 ranges leave a cluster of eight behind from about 30 blocks a CTA: 3x3 convs of one to four tiles,
+// us of a call, 24 blocks 36.8 / 36.6 and 44.1 / 44.9, 36 blocks 41.8 / 39.7 and 51.9 / 49.9.
 // Returns the CTAs per tile along K (1, 2, 4 or 8; 0: take the persistent kernel).
 int choose_unit(int auto_tile, long long M, int N, int batch, int num_kb)
 {
@@ -215,7 +217,7 @@ int choose_unit(int auto_tile, long long M, int N, int batch, int num_kb)
     if (tiles > 2 * SMS) return 0;
     int s = 1;
     while (s < 8 && tiles * s * 2 <= SMS && num_kb >= s * 4) s *= 2;
-    return num_kb > MAX_KB * s ? 0 : s;
+    return num_kb > (tiles * 16 <= SMS ? MAX_KB / 2 : MAX_KB) * s ? 0 : s;
 }
 
 // Whether the final output of `p` can be produced by the split-K reduce kernel (float path, 16-byte rows).
@@ -785,7 +787,11 @@ int run_conv_nchw(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvP
 // A one-wave fp32 product of caller tensors with tf32 operands, read where they lie: D = A * B^T with A [batch][M][K] and B
 // [batch][N][K], or [batch][K][N] (`b_kn`).  Rows of whole 16-byte pieces come by TMA; others, and a [K][N] operand, by plain
 // loads, which keep up only over a short K range: at most RAW_PLAIN_KB blocks a CTA.  Saves the packing kernels, their launches
-// and their passes over memory: Gemm 256 x 2048 x 1000 37.1 -> 35.8 us a call, MatMul 24 x 197 x 64 x 197 30.7 -> 29.5.
+// and their passes over memory: Gemm 256 x 2048 x 1000 37.1 -> 35.8 us a call, MatMul 24 x 197 x 64 x 197 30.7 -> 29.5.  The
+// rounding pass through shared memory takes about 0.5 us a K block of a CTA, the packing about 4 us and 0.43 us a megabyte of the
+// operands: in place up to 8 blocks and one more for every 1.2 MB.  us a call, in place / packed: 27 x K x 64 8 blocks (0.7 MB) 27.2
+// / 26.7, 24 blocks 40.5 / 32.1; 108 x K x 1758 16 blocks (15 MB) 37.1 / 39.7, 32 blocks (31 MB) 50.3 / 52.7; 1004 x K x 640
+// 8 blocks (1.7 MB) 26.8 / 26.9, 32 blocks (6.7 MB) 47.3 / 39.5.
 // Returns ONE_OK, an error, or 1 when the call is not of this form (the caller packs the operands): an output that shares memory
 // with an operand is not, since some CTAs still read what others have overwritten.
 constexpr int RAW_PLAIN_KB = 8;
@@ -804,7 +810,8 @@ int run_raw(one_ctx *ctx, int kind, const float *A, const float *B, int b_kn, lo
     u.a_ld = (K & 3) || (reinterpret_cast<uintptr_t>(A) & 15) ? 1 : 0;
     u.b_ld = b_kn ? 2 : ((K & 3) || (reinterpret_cast<uintptr_t>(B) & 15) ? 1 : 0);
     u.splits = choose_unit(!valid_tile(t_tile_n), M, N, batch, num_kb);
-    if (!u.splits || ((u.a_ld || u.b_ld) && (num_kb + u.splits - 1) / u.splits > RAW_PLAIN_KB)) return 1;
+    const long long limit = RAW_PLAIN_KB + (u.a_ld || u.b_ld ? 0 : (long long)(nb * (M + N) * K * 4 / 1200000));
+    if (!u.splits || (num_kb + u.splits - 1) / u.splits > limit) return 1;
     IgemmParams p;
     memset(&p, 0, sizeof(p));
     p.M = (int)M; p.N = N; p.num_kb = num_kb; p.slab_bytes = slab_bytes; p.slab_elems = slab_bytes / 4;

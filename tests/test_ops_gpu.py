@@ -779,3 +779,16 @@ def test_many_tiles_into_the_reference_layout(ops, oracle_mod, OC):
     assert_close(y, oracle_mod.conv_f32(x, w, b, (1, 1), (0,) * 4, abi.LEAKYRELU), str(OC))
     y8 = _np(ops.conv(x, w8, b32, act=abi.RELU, int8=(0.01, aux)))
     assert np.array_equal(y8, oracle_mod.conv_s8(x, w8, b32, aux, 0.01, (1, 1), 0, abi.RELU)[0])
+
+
+# one tile of 8 CTAs: 8 blocks a CTA and one more; more bytes to pack, more blocks
+@pytest.mark.parametrize("M,N,K,packed", [(70, 60, 8 * 8 * 32, False), (70, 60, 8 * 8 * 32 + 4, True), (100, 640, 16 * 8 * 32, False)])
+def test_operands_read_in_place_up_to_a_number_of_k_blocks(ops, oracle_mod, M, N, K, packed):
+    rng = np.random.default_rng(K)
+    a, w, b = rng.standard_normal((M, K)).astype(np.float32), (rng.standard_normal((N, K)) * 0.05).astype(np.float32), rng.standard_normal(N).astype(np.float32)
+    L = capi.lib()
+    ops.gemm(a, w, b)
+    before = L.one_cuda_launch_count()
+    y = _np(ops.gemm(a, w, b))
+    assert (L.one_cuda_launch_count() - before > 1) == packed
+    assert_close(y, oracle_mod.gemm(a, w, b), str(K))
