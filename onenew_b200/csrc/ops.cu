@@ -208,7 +208,8 @@ int run_split(one_ctx *ctx, int kind, int bn, const CUtensorMap &tmA, const CUte
 // kernel cuts them into 16 ranges leave a cluster of eight behind from about 30 blocks a CTA: 3x3 convs of one to four tiles,
 // us of a call, 24 blocks 36.8 / 36.6 and 44.1 / 44.9, 36 blocks 41.8 / 39.7 and 51.9 / 49.9.
 // Returns the CTAs per tile along K (1, 2, 4 or 8; 0: take the persistent kernel).
-int choose_unit(int auto_tile, long long M, int N, int batch, int num_kb)
+// `splittable`: the persistent kernel could split K over scratch planes instead.
+int choose_unit(int auto_tile, long long M, int N, int batch, int num_kb, bool splittable)
 {
     if (!auto_tile || t_split_k != 0) return 0;
     const long long tiles = ((M + 127) / 128) * ((N + UNIT_BN - 1) / UNIT_BN) * (batch > 0 ? batch : 1);
@@ -217,7 +218,13 @@ int choose_unit(int auto_tile, long long M, int N, int batch, int num_kb)
     if (tiles > 2 * SMS) return 0;
     int s = 1;
     while (s < 8 && tiles * s * 2 <= SMS && num_kb >= s * 4) s *= 2;
-    return num_kb > (tiles * 16 <= SMS ? MAX_KB / 2 : MAX_KB) * s ? 0 : s;
+    return num_kb > (splittable && tiles * 16 <= SMS ? MAX_KB / 2 : MAX_KB) * s ? 0 : s;
+}
+
+// What the two-pass split asks of a product into rows of its own (the rest is the caller's alignment, see split_eligible).
+bool splittable(const one_ctx *ctx, int kind, int N, int batch, const void *bias)
+{
+    return kind != KIND_I8 && batch == 0 && N % 4 == 0 && (reinterpret_cast<uintptr_t>(bias) & 15) == 0 && ctx->allow_split;
 }
 
 // Whether the final output of `p` can be produced by the split-K reduce kernel (float path, 16-byte rows).
@@ -563,7 +570,7 @@ int run_conv(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvPlan &
     UnitParams u;
     memset(&u, 0, sizeof(u));
     u.b_const = io.w_const; u.nchw_hw = io.y_nchw ? g.OH * g.OW : 0;
-    if ((u.splits = choose_unit(pl.auto_tile, M, g.OC, 0, pl.num_kb)) && unit_epilogue(pl.kind, p, u) >= 0) {
+    if ((u.splits = choose_unit(pl.auto_tile, M, g.OC, 0, pl.num_kb, splittable(ctx, pl.kind, g.OC, 0, io.bias))) && unit_epilogue(pl.kind, p, u) >= 0) {
         CUtensorMap tmU;
         rc = make_tmap_tiled(&tmU, kind_tm(pl.kind), io.w, pl.w_pitch, g.OC, 0, (uint64_t)pl.w_pitch * pl.es, 0, pl.slab_elems, UNIT_BN, pl.slab_bytes);
         if (rc != ONE_OK) return rc;
@@ -683,7 +690,7 @@ int run_gemm(one_ctx *ctx, int kind, const void *A, int a_pitch, const void *B, 
     UnitParams u;
     memset(&u, 0, sizeof(u));
     u.b_const = prepared;
-    const bool unit = (u.splits = choose_unit(auto_tile, M, N, batch, p.num_kb)) && unit_epilogue(kind, p, u) >= 0;
+    const bool unit = (u.splits = choose_unit(auto_tile, M, N, batch, p.num_kb, splittable(ctx, kind, N, batch, bias))) && unit_epilogue(kind, p, u) >= 0;
     if (tmB_cached && !unit) tmB = *tmB_cached;
     else {
         rc = make_tmap_tiled(&tmB, kind_tm(kind), B, K, N, batch, (uint64_t)b_pitch * es, (uint64_t)b_bstride * es,
@@ -765,10 +772,11 @@ int run_conv_nchw(one_ctx *ctx, const ConvGeom &g, const ConvEpi &e, const ConvP
     const size_t out_bytes = (size_t)M * g.OC * 4;
     io.out_mode = OUT_F32;
     const bool shared = (io.bias && overlap(out, out_bytes, io.bias, (size_t)g.OC * 4)) || (e.act == SILU && overlap(out, out_bytes, io.lut, 8192 * 4));
-    const bool unit = choose_unit(pl.auto_tile, M, g.OC, 0, pl.num_kb) && !(e.act == SILU && (reinterpret_cast<uintptr_t>(io.lut) & 15));
+    const bool can = splittable(ctx, pl.kind, g.OC, 0, io.bias);
+    const bool unit = choose_unit(pl.auto_tile, M, g.OC, 0, pl.num_kb, can) && !(e.act == SILU && (reinterpret_cast<uintptr_t>(io.lut) & 15));
     int per;
-    const bool split = !unit && pl.kind != KIND_I8 && g.OC % 4 == 0 && (reinterpret_cast<uintptr_t>(io.bias) & 15) == 0 &&
-                       ((!pl.cta2 && pl.mh == 1 && pl.nw == 8) || plain_for_split(pl.auto_tile, pl.kind)) && choose_split(ctx, M, g.OC, pl.bn, pl.num_kb, &per) > 1;
+    const bool split = !unit && can && ((!pl.cta2 && pl.mh == 1 && pl.nw == 8) || plain_for_split(pl.auto_tile, pl.kind)) &&
+                       choose_split(ctx, M, g.OC, pl.bn, pl.num_kb, &per) > 1;
     const bool rows = !unit && ((g.OC % 32 == 0 && (reinterpret_cast<uintptr_t>(io.bias) & 15) == 0) || (g.OC > 128 && out_bytes >= (size_t(16) << 20)));
     void *yh = shared || split || rows ? ws_alloc(ctx, out_bytes) : nullptr;
     if (shared && !yh) return fail(ONE_ERR_NOMEM, "Conv: workspace too small for the NHWC output");
@@ -809,7 +817,7 @@ int run_raw(one_ctx *ctx, int kind, const float *A, const float *B, int b_kn, lo
     if (batch) { u.a_bstride = M * K; u.b_bstride = (long long)N * K; }
     u.a_ld = (K & 3) || (reinterpret_cast<uintptr_t>(A) & 15) ? 1 : 0;
     u.b_ld = b_kn ? 2 : ((K & 3) || (reinterpret_cast<uintptr_t>(B) & 15) ? 1 : 0);
-    u.splits = choose_unit(!valid_tile(t_tile_n), M, N, batch, num_kb);
+    u.splits = choose_unit(!valid_tile(t_tile_n), M, N, batch, num_kb, splittable(ctx, kind, N, batch, bias));
     const long long limit = RAW_PLAIN_KB + (u.a_ld || u.b_ld ? 0 : (long long)(nb * (M + N) * K * 4 / 1200000));
     if (!u.splits || (num_kb + u.splits - 1) / u.splits > limit) return 1;
     IgemmParams p;

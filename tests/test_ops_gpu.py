@@ -792,3 +792,24 @@ def test_operands_read_in_place_up_to_a_number_of_k_blocks(ops, oracle_mod, M, N
     y = _np(ops.gemm(a, w, b))
     assert (L.one_cuda_launch_count() - before > 1) == packed
     assert_close(y, oracle_mod.gemm(a, w, b), str(K))
+
+
+def test_long_k_that_the_scratch_planes_cannot_take_stays_in_clusters(ops, oracle_mod):
+    """Batched products, ragged widths and int8 convs are not split over scratch planes: the one-wave kernel keeps them."""
+    rng = np.random.default_rng(31)
+    a3, b3 = rng.standard_normal((2, 60, 9000)).astype(np.float32), (rng.standard_normal((2, 9000, 64)) * 0.02).astype(np.float32)
+    y = _np(ops.matmul(a3, b3))
+    assert capi.last_form() == "tile=128x64 split=8 unit"
+    assert_close(y, np.matmul(a3.astype(np.float64), b3).astype(np.float32), "batched")
+    a, w, b = rng.standard_normal((60, 9000)).astype(np.float32), (rng.standard_normal((63, 9000)) * 0.02).astype(np.float32), rng.standard_normal(63).astype(np.float32)
+    y = _np(ops.gemm(a, w, b))
+    assert capi.last_form() == "tile=128x64 split=8 unit"
+    assert_close(y, oracle_mod.gemm(a, w, b), "ragged")
+    y = _np(ops.gemm(a, w[:60], b[:60]))
+    assert capi.last_form() == "tile=128x64 split=16"
+    assert_close(y, oracle_mod.gemm(a, w[:60], b[:60]), "rows of whole pieces")
+    x, cw = rng.uniform(-1, 1, (1, 768, 9, 9)).astype(np.float32), (rng.standard_normal((32, 768, 7, 7)) * 0.05).astype(np.float32)
+    w8, b32, aux = oracle_mod.quant_weight_bias(cw, b[:32])
+    y = _np(ops.conv(x, w8, b32, pads=(3,) * 4, act=abi.RELU, int8=(0.01, aux)))
+    assert capi.last_form() == "tile=128x64 split=8 unit"
+    assert np.array_equal(y, oracle_mod.conv_s8(x, w8, b32, aux, 0.01, (1, 1), 3, abi.RELU)[0])
