@@ -176,7 +176,9 @@ ONE_API int one_cuda_set_tile_n(int bn);
  * allows it (output rows and bias of whole 16-byte pieces, scratch for the planes, and no tile code above 1000
  * asked for).  Only the float paths split that way; results do not depend on scheduling.  With 0, and no tile
  * override, a launch whose 128 x 64 tiles are all resident at once runs one tile per CTA instead, its K range
- * shared by a cluster of up to eight CTAs; 1 therefore also gives sums that do not depend on the batch. */
+ * shared by a cluster of up to eight CTAs.  1 gives TF32 and int8 results that do not depend on the batch; with
+ * 16-bit storage a fused residual is added before or after the bias according to the tile, which the batch decides
+ * (bit 3 of one_cuda_set_epilogue_mode off: always after it). */
 ONE_API int one_cuda_set_split_k(int splits);
 /* The same choice for one prepared operator (0: follow the calling thread's setting); used by the tile search. */
 ONE_API int one_cuda_packed_set_split(one_packed *op, int splits);

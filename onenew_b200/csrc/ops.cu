@@ -113,9 +113,11 @@ inline int kind_of_prec(int prec) { return prec == ONE_PREC_BF16 ? KIND_BF16 : (
 inline bool valid_prec(int prec) { return prec == ONE_PREC_TF32 || prec == ONE_PREC_BF16 || prec == ONE_PREC_F16; }
 inline int kind_out16(int kind) { return kind == KIND_F16 ? OUT_F16 : OUT_BF16; }   // the kind's own 16-bit output mode
 // How the tiles of width `bn` are walked when the library chooses (`taps`: a filter of several positions; 0 a plain product;
-// c_slabs: K blocks per filter position).  Every form gives the same sums; they differ in what bounds a launch of many tiles.
-// Until now only a tile search chose them.  Whole networks, us, single CTAs -> this rule: int8 backbone of 64 images
-// 1955 -> 1625, ResNet-50 fp16 256 images 4837 -> 4535, ViT-Tiny 256 images 3555 -> 3485, ResNet-50 TF32 61 images equal.
+// c_slabs: K blocks per filter position).  They differ in what bounds a launch of many tiles.  Every form adds a tile's products
+// in the same order; only a 16-bit residual, which plain 256-wide tiles add before the bias by the tensor core (see res_mma) and
+// every other form after it, is rounded in another order.  Whole networks, us, single CTAs -> this rule, the sides timed in turn:
+// int8 backbone of 64 images 1955 -> 1625, ResNet-50 fp16 256 images 4829 -> 4721, ViT-Tiny 256 images 3650 -> 3537 (attention's
+// second softmax warp among it), ResNet-50 TF32 61 images equal.
 //  * 64 wide: operand traffic and barrier hand-overs -- two 128-row halves against one tile of B.  TF32 products of few K
 //    blocks are bound by HBM instead and stay plain.
 //  * 128 wide, 3x3 filters of enough channels: the same; from about a wave on, since halves also shorten a ragged last wave.
@@ -1317,9 +1319,15 @@ static int prepare_gemm(one_packed *op, bool is_gemm, BUFFER_INFO_S *params, BUF
         long long rows = 1;
         for (int i = 0; i < a0->dim_num_of_shapes - 1 && i < SHAPE_LEN; ++i) rows *= a0->shapes[i];
         op->bn = refine_tile(pick_bn(op->N, rows), op->kind, rows, op->N, (int)(((long long)op->K * es + 127) / 128), false, 1);
-        // ViT-Tiny's widths: pairs when the rows are many (qkv, fc2)
-        if (op->bn == 192 && !valid_tile(t_tile_n) && g_cta_pairs.load(std::memory_order_relaxed) && op->kind == KIND_TF32 && (long long)op->K * es >= 6 * 128 &&
-            (rows + 127) / 128 * ((op->N + 191) / 192) >= 2 * 148)
+        // 192 wide in TF32: pairs of CTAs from 5 K blocks and two waves of row tiles on.  The line is drawn by rows and not by
+        // tiles because a network's layers share its rows: where some of them run as pairs and others do not, the changes from
+        // one to the other cost more than the pairs save.  ViT of width 192, us a pass, none / all that have two waves of tiles /
+        // this rule: 197 tokens x 97 images (150 row tiles) 1758 / 1805 / 1758, 128 (197) 1972 / 2100 / 1972, 160 (247) 2419 /
+        // 2473 / 2419, 192 (296) 2640 / 2620 / 2620, 256 (394) 3527 / 3495 / 3495, 400 (616) 5270 / 5247 / 5247; 65 tokens x 300
+        // (153) 1768 / 1819 / 1768, 600 (305) 3024 / 2992 / 2992; width 384 x 64 images (99) 2528 / 2566 / 2528, 110 (170) 3733 /
+        // 3689 / 3733.  One product alone gains from 5 K blocks on: 2346 tiles 4 66.2 / 67.7, 5 75.5 / 69.3, 6 75.7 / 72.4.
+        if (op->bn == 192 && !valid_tile(t_tile_n) && g_cta_pairs.load(std::memory_order_relaxed) && op->kind == KIND_TF32 &&
+            (long long)op->K * es >= 5 * 128 && (rows + 127) / 128 >= 2 * 148)
             op->bn = 1192;
         op->auto_tile = !valid_tile(t_tile_n);
     }
