@@ -35,7 +35,7 @@ __device__ __forceinline__ float apply_act(float v, int act, float p0, float p1,
     case 3:
         if (v < -8.0f) return 0.f;
         if (v >= 8.0f) return v;
-        if (v >= -8.0f && v < 8.0f) return lut[(int)__fmul_rn(__fadd_rn(v, 8.0f), 512.0f)];
+        if (v >= -8.0f && v < 8.0f) return __ldg(lut + (int)__fmul_rn(__fadd_rn(v, 8.0f), 512.0f));
         return v;
     case 4: {
         float t = v > p0 ? v : p0;

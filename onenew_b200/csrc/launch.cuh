@@ -74,7 +74,8 @@ template <typename P> __device__ __forceinline__ void launder(P &p) { asm volati
 // Start of a kernel launched by launch_k: the next launch may be placed, this one waits until the previous kernel
 // has completed and its writes are visible.  The pointers the kernel reads through are passed here so that the
 // compiler cannot turn loads through a `const __restrict__` pointer into read-only ones (ld.global.nc), or move them above the
-// wait: the wait does not order read-only loads.  So no __ldg of what an earlier kernel may have written either.
+// wait: the wait does not order read-only loads.  So no __ldg of what an earlier kernel may have written either (an activation
+// table never is: a prepared operator's copy, or complete before the call, see FirstLaunchPlain).
 template <typename... P> __device__ __forceinline__ void pdl_entry(P &...ptrs)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
