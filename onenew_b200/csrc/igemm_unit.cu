@@ -174,17 +174,19 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const int col = n0 + c0 + chunk * 4, nvalid = p.N - col;        // this lane's four columns in a row-major output
     const bool f16 = p.out_mode == OUT_F16;
     alignas(16) float cst_[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    // (The caller's tensors may have been written by an earlier kernel of the stream.  Plain loads here and below: a read-only
-    // one, __ldg, is not ordered by the wait -- one behind a conditional wait was seen to run ahead of it.)
+    // Plain loads here and below: what an earlier kernel of the stream may have written is read after the wait, and a read-only
+    // load, __ldg, is not ordered by it -- one behind a conditional wait was seen to run ahead of it.
     const float *bias = reinterpret_cast<const float *>(p.bias);
-    if (!u.b_const && p.pdl) pdl_wait();
-    if (ROWS && nvalid > 0) {
+    auto load_constants = [&]() {
+        if (ROWS && nvalid > 0) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            if (bias) cst_[e] = bias[col + e];
-            if (KIND == KIND_I8) cst_[4 + e] = p.coeff[col + e];
+            for (int e = 0; e < 4; ++e) {
+                if (bias) cst_[e] = bias[col + e];
+                if (KIND == KIND_I8) cst_[4 + e] = p.coeff[col + e];
+            }
         }
-    }
+    };
+    if (u.b_const) load_constants();
 
     const bool tma_a = !RAW || u.a_ld == 0, tma_b = !RAW || u.b_ld == 0;
     const uint32_t tx = (tma_a ? a_slab : 0u) + (tma_b ? b_slab : 0u);
@@ -260,6 +262,7 @@ unit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     } else {
         if (p.pdl) pdl_wait();
     }
+    if (!u.b_const) load_constants();   // (behind the first loads: ahead of them they cost Gemm 256 x 2048 x 1000 0.3 us of 35)
     if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         const uint32_t idesc = make_idesc<KIND>(A_ROWS, BN) & ((KIND == KIND_BF16 && p.ab_f16) ? ~((7u << 7) | (7u << 10)) : ~0u);
